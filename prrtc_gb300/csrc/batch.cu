@@ -106,6 +106,7 @@ struct prrtc_batch {
     std::vector<int> num_goals;
     // device
     void *blob = nullptr;          // cfg pool | env pool | descs | slots | outs | counters | path pool
+    char *grids = nullptr;         // clearance grids of the queries that bring host obstacles
     Arena *arena = nullptr;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -114,6 +115,11 @@ struct prrtc_batch {
     unsigned long long t0 = 0;     // device clock at the last run's start (first warp)
     bool ran = false;
 };
+
+// cells of a query's own clearance grid (135 KB; 8-10 cm cells on the
+// tabletop and shelf scenes), and the most memory a batch spends on them
+static constexpr int kBatchCells = 4096;
+static constexpr size_t kGridBytes = (size_t)8 << 30;
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -175,6 +181,8 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
             const Env *e = reinterpret_cast<const Env *>(q.env);
             descs[i].env = e->dev;
             descs[i].env_n = e->counts;
+            descs[i].grid = e->grid;
+            descs[i].build = 0;
         } else {
             const prrtc_env_desc &e = *q.env_desc;
             env_rec_off[i] = (int)envs.size();
@@ -228,14 +236,30 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
         delete b;
         return c->fail(PRRTC_ENOMEM, "batch_create: cannot allocate %zu bytes", off);
     }
+    // queries that bring host obstacles get a clearance grid of their own, if
+    // there is room for them (without it the checker tests every obstacle)
+    size_t own_envs = 0, own = 0;
+    for (int i = 0; i < n; i++) own_envs += env_rec_off[i] >= 0 && descs[i].env_n.obstacles() > 0;
+    const size_t grid_bytes = env_grid_bytes(kBatchCells);
+    if (own_envs > 0 && own_envs * grid_bytes <= kGridBytes && cudaMalloc(&b->grids, own_envs * grid_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        b->grids = nullptr;
+    }
     char *base = static_cast<char *>(b->blob);
     float4 *env_dev = reinterpret_cast<float4 *>(base + o_env);
     for (int i = 0; i < n; i++)
-        if (env_rec_off[i] >= 0) descs[i].env = env_dev + env_rec_off[i];
+        if (env_rec_off[i] >= 0) {
+            descs[i].env = env_dev + env_rec_off[i];
+            const bool grid = b->grids && descs[i].env_n.obstacles() > 0;
+            descs[i].grid = grid ? reinterpret_cast<const EnvGrid *>(b->grids + grid_bytes * own++) : nullptr;
+            descs[i].build = grid;
+        }
     if ((s = ensure_halton_bases(c, b->lanes * max_attempts)) ||
         (s = c->cuda(cudaMemcpyAsync(base + o_cfg, cfg.data(), cfg.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream), "batch upload")) ||
         (!envs.empty() && (s = c->cuda(cudaMemcpyAsync(env_dev, envs.data(), envs.size() * sizeof(float4), cudaMemcpyHostToDevice, c->stream), "batch upload"))) ||
         (s = c->cuda(cudaMemcpyAsync(base + o_desc, descs.data(), n * sizeof(BatchQueryDesc), cudaMemcpyHostToDevice, c->stream), "batch upload")) ||
+        (own && (s = c->cuda(launch_env_grids(reinterpret_cast<const BatchQueryDesc *>(base + o_desc), n, BatchQueryDesc{},
+                                              kBatchCells, c->stream), "batch grids"))) ||
         (s = take_arena(c, D, cap, slots, &b->arena)) ||
         (s = c->cuda(cudaEventCreate(&b->ev0), "event")) || (s = c->cuda(cudaEventCreate(&b->ev1), "event")) ||
         (s = c->cuda(cudaStreamSynchronize(c->stream), "batch upload"))) {
@@ -468,6 +492,7 @@ extern "C" prrtc_status prrtc_batch_free(prrtc_ctx *ctx, prrtc_batch *b)
         if (b->ev0) cudaEventDestroy(b->ev0);
         if (b->ev1) cudaEventDestroy(b->ev1);
         cudaFree(b->blob);
+        cudaFree(b->grids);
         give_back_arena(c, b->arena);
     }
     delete b;

@@ -55,6 +55,7 @@ struct alignas(16) WarpScratch {
     int pend_t[32], pend_i[32], pend_it[32];
     float pend_d[32];
     unsigned long long env_bar;   // mbarrier of the bulk copies that stage the obstacle records
+    EnvGrid grid;                 // the header of the query's clearance grid
     int bad;
 };
 
@@ -560,6 +561,7 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
     bool trapped = false;   // this warp's last round on its slot was rejected early in full
     unsigned idle = 0;
     const float4 *staged = nullptr;   // the global records now in W_env
+    const EnvGrid *staged_grid = nullptr;   // the grid whose header is in W.grid
     const unsigned env_bar = (unsigned)__cvta_generic_to_shared(&W.env_bar);
     unsigned env_phase = 0;           // parity of W.env_bar's next phase
     if (lane == 0) {
@@ -758,7 +760,15 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
             }
             envp = W_env;
         }
-        CheckCtx ctx{{envp, Qd.env_n}, P.pad, &W.bad};
+        if (Qd.grid && staged_grid != Qd.grid) {
+            __syncwarp();
+            constexpr int words = sizeof(EnvGrid) / sizeof(int);
+            for (int i = lane; i < words; i += 32)
+                reinterpret_cast<int *>(&W.grid)[i] = __ldg(reinterpret_cast<const int *>(Qd.grid) + i);
+            __syncwarp();
+            staged_grid = Qd.grid;
+        }
+        CheckCtx ctx{{envp, Qd.env_n, Qd.grid ? &W.grid : nullptr}, P.pad, &W.bad};
         SharedCheckCtx sctx{ctx, W_frames + lane};
         // every point of an edge through the robot's checker, frames where P says
         auto validate = [&]() {

@@ -259,6 +259,10 @@ prrtc_status prrtc_robot_limits(prrtc_robot robot, float *scale, float *offset)
     return PRRTC_OK;
 }
 
+// cells of an uploaded environment's clearance grid (0.8 MB): about 5 cm
+// cells on the tabletop and shelf scenes
+static constexpr int kEnvCells = 24576;
+
 prrtc_status prrtc_env_upload(prrtc_ctx *ctx, const prrtc_env_desc *d, prrtc_env **out)
 {
     Ctx *c = Ctx::of(ctx);
@@ -284,14 +288,23 @@ prrtc_status prrtc_env_upload(prrtc_ctx *ctx, const prrtc_env_desc *d, prrtc_env
     e->num_cylinders = d->num_cylinders;
     if (!e->host.empty()) {
         cudaSetDevice(c->device);
-        if (cudaMalloc(&e->dev, e->host.size() * sizeof(float4)) != cudaSuccess) {
+        const size_t rec_bytes = e->host.size() * sizeof(float4);
+        // room for the grid if there is any (without it the checker tests every obstacle)
+        bool grid = cudaMalloc(&e->dev, rec_bytes + env_grid_bytes(kEnvCells)) == cudaSuccess;
+        if (!grid && (cudaGetLastError(), cudaMalloc(&e->dev, rec_bytes) != cudaSuccess)) {
             cudaGetLastError();
             delete e;
             return c->fail(PRRTC_ENOMEM, "env_upload: cudaMalloc failed");
         }
-        prrtc_status s = c->cuda(cudaMemcpy(e->dev, e->host.data(), e->host.size() * sizeof(float4), cudaMemcpyHostToDevice),
-                                 "env_upload copy");
-        if (s) {
+        BatchQueryDesc d{};
+        d.env = e->dev;
+        d.env_n = e->counts;
+        d.grid = e->grid = grid ? reinterpret_cast<const EnvGrid *>(e->dev + e->host.size()) : nullptr;
+        d.build = 1;
+        prrtc_status s;
+        if ((s = c->cuda(cudaMemcpyAsync(e->dev, e->host.data(), rec_bytes, cudaMemcpyHostToDevice, c->stream), "env_upload copy")) ||
+            (grid && (s = c->cuda(launch_env_grids(nullptr, 1, d, kEnvCells, c->stream), "env_upload grid"))) ||
+            (s = c->cuda(cudaStreamSynchronize(c->stream), "env_upload"))) {
             cudaFree(e->dev);
             delete e;
             return s;
@@ -328,7 +341,7 @@ prrtc_status prrtc_validate_configs(prrtc_ctx *ctx, prrtc_robot robot, const prr
     prrtc_status s;
     if ((s = c->device_view(q, sizeof(float) * ops->dof * n, 0, true, &dq))) return s;
     if ((s = c->device_view(out_free, n, 1, false, &dout))) return s;
-    LaunchEnv le{e->dev, e->counts, c->sms, c->work_dev};
+    LaunchEnv le{e->dev, e->counts, c->sms, c->work_dev, e->grid};
     cudaEventRecord(c->kev[0], c->stream);
     if ((s = c->cuda(ops->validate_configs(le, (const float *)dq, n, (uint8_t *)dout, c->stream), "validate_configs launch"))) return s;
     cudaEventRecord(c->kev[1], c->stream);
@@ -366,7 +379,7 @@ prrtc_status prrtc_sample_goals(prrtc_ctx *ctx, prrtc_robot robot, const prrtc_e
     prrtc_robot_limits(robot, gq.scale, gq.offset);
     uint8_t *flags = static_cast<uint8_t *>(c->scratch(1, (size_t)tries));
     if (!flags) return c->fail(PRRTC_ENOMEM, "sample_goals: %lld flags", (long long)tries);
-    LaunchEnv le{e->dev, e->counts, c->sms, nullptr};
+    LaunchEnv le{e->dev, e->counts, c->sms, nullptr, e->grid};
     prrtc_status s;
     if ((s = c->cuda(ops->goal_flags(le, gq, flags, c->stream), "sample_goals launch"))) return s;
     c->launches++;
@@ -399,7 +412,7 @@ prrtc_status prrtc_validate_edges(prrtc_ctx *ctx, prrtc_robot robot, const prrtc
     if ((s = c->device_view(a, cb, 0, true, &da))) return s;
     if ((s = c->device_view(b, cb, 2, true, &db))) return s;
     if ((s = c->device_view(out_free, n, 1, false, &dout))) return s;
-    LaunchEnv le{e->dev, e->counts, c->sms, c->work_dev};
+    LaunchEnv le{e->dev, e->counts, c->sms, c->work_dev, e->grid};
     cudaEventRecord(c->kev[0], c->stream);
     if ((s = c->cuda(ops->validate_edges(le, (const float *)da, (const float *)db, n, granularity, (uint8_t *)dout, c->stream),
                      "validate_edges launch")))

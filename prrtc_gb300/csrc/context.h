@@ -11,7 +11,8 @@ namespace prrtc {
 
 struct Env {
     EnvCounts counts{};
-    float4 *dev = nullptr;           // packed records on the device
+    float4 *dev = nullptr;           // packed records on the device, followed by the clearance grid
+    const EnvGrid *grid = nullptr;
     std::vector<float4> host;        // the same records on the host
     uint32_t num_cylinders = 0;      // accepted, never checked (as the reference)
 };

@@ -29,11 +29,35 @@ struct LeafPair {
 struct EnvCounts {
     int ns, nc, nzc, ncb, nzb;
     __host__ __device__ int records() const { return ns + 2 * nc + 2 * nzc + 4 * ncb + 4 * nzb; }
+    __host__ __device__ int obstacles() const { return ns + nc + nzc + ncb + nzb; }
 };
+
+// Clearance grid of an environment, built on the device when the environment
+// is uploaded (env_grid.cu).  A box around the obstacles is cut into cells;
+// per cell the grid holds a lower bound of the distance from any point of
+// the cell to the nearest obstacle (near), and the bounds and numbers of the
+// 15 nearest ones (list), so a sphere in free space costs one byte read
+// instead of a test against every obstacle, and one near obstacles tests
+// only those it can touch.  Bounds are in units of 1 / kGridUnit metres,
+// rounded down, 255 for "at least that far".  They bound the reference's
+// tests themselves (env_grid.cu says how), so skipping an obstacle never
+// changes a verdict.
+struct EnvGrid {
+    float inv[3], off[3];   // a point's cell along an axis: round(p * inv + off)
+    int n[3];               // cells per axis, x fastest; 0: the environment has no grid cells
+    int cost;               // FLOPs of a sphere tested against every obstacle
+    float lo[3], hi[3];     // box around the obstacles; lo > hi: the grid is not to be used
+    const uint8_t *near_;   // per cell: bound of the nearest obstacle
+    const uint4 *list;      // per cell two uint4: 16 bounds (15 obstacles, by number; then the next one's), 16 numbers
+};
+constexpr float kGridUnit = 512.0f;
+constexpr int kGridListed = 15;        // obstacles listed per cell
+constexpr int kGridMaxObstacles = 255; // numbers are bytes; 255 marks an unused entry
 
 struct EnvView {
     const float4 *rec;   // records (shared memory once staged)
     EnvCounts n;
+    const EnvGrid *grid = nullptr;
 };
 
 // Copy a packed environment into shared memory (all threads of the block
@@ -93,6 +117,17 @@ __device__ __forceinline__ void stage_env_bulk(float4 *smem, const float4 *__res
         for (int i = 0; i < kBulkPolls && !done; i++) done = bulk_phase_done(bar, 0u);
         __syncthreads();
     }
+}
+
+// Copy a grid's header into shared memory (all threads of the block
+// participate; caller synchronises); returns the copy, or null for none.
+__device__ __forceinline__ const EnvGrid *stage_grid(EnvGrid *smem, const EnvGrid *__restrict__ g)
+{
+    constexpr int words = sizeof(EnvGrid) / sizeof(int);
+    if (!g) return nullptr;
+    for (int i = threadIdx.x; i < words; i += blockDim.x)
+        reinterpret_cast<int *>(smem)[i] = __ldg(reinterpret_cast<const int *>(g) + i);
+    return smem;
 }
 
 // ---- the reference's primitive tests (src/planning/utils.cuh:58-209) ------
@@ -157,7 +192,7 @@ constexpr int kFlopSphere = 11, kFlopCapsule = 26, kFlopZCapsule = 16, kFlopCubo
 // Spheres, capsules and cuboids are tested two at a time (independent
 // dependency chains, one branch); on a hit the count stops at the first
 // hitting test, so verdicts and counts are the reference's, in its order.
-static __device__ __noinline__ int env_hit(const EnvView e, float x, float y, float z, float r)
+static __device__ __noinline__ int env_hit_all(const EnvView e, float x, float y, float z, float r)
 {
     const float4 *p = e.rec;
     int w = 0, i = 0;
@@ -205,6 +240,127 @@ static __device__ __noinline__ int env_hit(const EnvView e, float x, float y, fl
         if (hit_z_cuboid(p[4 * i], p[4 * i + 1], p[4 * i + 2], x, y, z, rsq)) return 2 * w + 1;
     }
     return 2 * w;
+}
+
+// FLOPs of one sphere against obstacles 0 .. k-1, in the reference's order
+__device__ __forceinline__ int env_cost(const EnvCounts &n, int k)
+{
+    const int a = min(k, n.ns);
+    k -= a;
+    const int b = min(k, n.nc);
+    k -= b;
+    const int c = min(k, n.nzc);
+    k -= c;
+    const int d = min(k, n.ncb);
+    return a * kFlopSphere + b * kFlopCapsule + c * kFlopZCapsule + d * kFlopCuboid + (k - d) * kFlopZCuboid;
+}
+
+// Sphere against obstacle k: 0 no hit, 1 hit, 2 too near contact to tell
+// here.  The distance is the reference test's; what is left to env_hit_all is
+// a band around contact wider than any rounding (coordinates are at most
+// kGridReach, so a distance's rounding is near 1e-5 m at most), so that
+// verdicts do not depend on how two copies of a formula are contracted.
+constexpr float kGridReach = 16.0f;
+__device__ __forceinline__ int near_test(const float4 *__restrict__ rec, const EnvCounts &n, int k, float x, float y,
+                                         float z, float r)
+{
+    float d2, rs;
+    if (k < n.ns) {
+        const float4 s = rec[k];
+        const float dx = x - s.x, dy = y - s.y, dz = z - s.z;
+        d2 = dx * dx + dy * dy + dz * dz;
+        rs = r + s.w;
+    } else if (k < n.ns + n.nc + n.nzc) {
+        const bool upright = k >= n.ns + n.nc;
+        const float4 *c = rec + n.ns + 2 * (k - n.ns);
+        const float4 a = c[0];
+        float4 v = c[1];
+        if (upright) v.x = v.y = 0.0f;
+        const float dot = (x - a.x) * v.x + (y - a.y) * v.y + (z - a.z) * v.z;
+        const float t = fmaxf(fminf(dot * v.w, 1.0f), 0.0f);
+        const float dx = x - (a.x + v.x * t), dy = y - (a.y + v.y * t), dz = z - (a.z + v.z * t);
+        d2 = dx * dx + dy * dy + dz * dz;
+        rs = r + a.w;
+    } else {
+        const bool upright = k >= n.ns + n.nc + n.nzc + n.ncb;
+        const float4 *c = rec + n.ns + 2 * (n.nc + n.nzc) + 4 * (k - n.ns - n.nc - n.nzc);
+        const float4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+        const float xs = x - c0.x, ys = y - c0.y, zs = z - c0.z;
+        const float u1 = c1.x * xs + c1.y * ys, u2 = c2.x * xs + c2.y * ys;
+        const float a1 = fmaxf(0.0f, fabsf(upright ? u1 : u1 + c1.z * zs) - c0.w);
+        const float a2 = fmaxf(0.0f, fabsf(upright ? u2 : u2 + c2.z * zs) - c1.w);
+        const float a3 = fmaxf(0.0f, fabsf(upright ? zs : c3.x * xs + c3.y * ys + c3.z * zs) - c2.w);
+        d2 = a1 * a1 + a2 * a2 + a3 * a3;
+        rs = r;
+    }
+    const float v = d2 - rs * rs, band = 1e-5f * (d2 + rs * rs) + 4e-5f * fabsf(rs);
+    return v > band ? 0 : v < -band ? 1 : 2;
+}
+
+// the cell of a point, -1 outside the cells (any NaN coordinate, too).  The
+// sum with 1.5 x 2^23 rounds to the nearest integer in the float's low bits,
+// at the FMA pipe's rate (a conversion instruction runs at a quarter of it).
+__device__ __forceinline__ int grid_cell(const EnvGrid &g, float x, float y, float z)
+{
+    constexpr float kMagic = 12582912.0f;
+    const unsigned ix = __float_as_uint(__fadd_rn(fmaf(x, g.inv[0], g.off[0]), kMagic)) - 0x4B400000u;
+    const unsigned iy = __float_as_uint(__fadd_rn(fmaf(y, g.inv[1], g.off[1]), kMagic)) - 0x4B400000u;
+    const unsigned iz = __float_as_uint(__fadd_rn(fmaf(z, g.inv[2], g.off[2]), kMagic)) - 0x4B400000u;
+    const bool in = ix < (unsigned)g.n[0] && iy < (unsigned)g.n[1] && iz < (unsigned)g.n[2];
+    return in ? (int)(ix + g.n[0] * (iy + g.n[1] * iz)) : -1;
+}
+
+// one bit per byte of w that is below t (both unsigned, t <= 255)
+__device__ __forceinline__ unsigned bytes_below(unsigned w, unsigned t4)
+{
+    return ((__vcmpltu4(w, t4) & 0x01010101u) * 0x01020408u) >> 24;
+}
+
+// Sphere against every obstacle by the clearance grid, result as env_hit's;
+// -1 where the grid cannot tell (no grid, a sphere larger than its bounds
+// reach, more than kGridListed obstacles near, a contact too near).
+__device__ __forceinline__ int grid_hit(const EnvView &e, float x, float y, float z, float r)
+{
+    const EnvGrid &g = *e.grid;
+    const float ra = fabsf(r);
+    const int none = 2 * g.cost;
+    const int cell = grid_cell(g, x, y, z);
+    if (cell < 0) {   // outside the cells: by the box around the obstacles (finite coordinates only)
+        const float dx = fmaxf(fmaxf(g.lo[0] - x, x - g.hi[0]), 0.0f), dy = fmaxf(fmaxf(g.lo[1] - y, y - g.hi[1]), 0.0f),
+                    dz = fmaxf(fmaxf(g.lo[2] - z, z - g.hi[2]), 0.0f);
+        const float rs = ra * 1.01f + 1e-3f;
+        const bool sure = g.lo[0] <= g.hi[0] && fabsf(x) + fabsf(y) + fabsf(z) < 1e4f;
+        return sure && dx * dx + dy * dy + dz * dz > rs * rs ? none : -1;
+    }
+    const int thr = __float2int_ru(ra * kGridUnit);
+    if (thr > 255) return -1;
+    if ((int)__ldg(g.near_ + cell) >= thr) return none;
+    const uint4 lb = __ldg(g.list + 2 * cell);
+    const unsigned t4 = (unsigned)thr * 0x01010101u;
+    unsigned m = bytes_below(lb.x, t4) & 15u;
+    m |= (bytes_below(lb.y, t4) & 15u) << 4;
+    m |= (bytes_below(lb.z, t4) & 15u) << 8;
+    m |= (bytes_below(lb.w, t4) & 15u) << 12;
+    if (m >> kGridListed) return -1;
+    const uint8_t *num = reinterpret_cast<const uint8_t *>(g.list + 2 * cell + 1);
+    while (m) {
+        const int k = __ldg(num + __ffs(m) - 1);
+        m &= m - 1;
+        const int h = near_test(e.rec, e.n, k, x, y, z, r);
+        if (h == 2) return -1;
+        if (h == 1) return 2 * env_cost(e.n, k + 1) + 1;
+    }
+    return none;
+}
+
+// Sphere against every obstacle: by the grid where there is one.  Every
+// obstacle for every sphere was two thirds of a check; 2^20 random
+// configurations on the Panda shelf scene (41 obstacles) take 1.01 ms instead
+// of 1.86, 200 003 Baxter ones among 72 obstacles 0.66 ms instead of 1.20.
+static __device__ __noinline__ int env_hit(const EnvView e, float x, float y, float z, float r)
+{
+    const int h = e.grid ? grid_hit(e, x, y, z, r) : -1;
+    return h >= 0 ? h : env_hit_all(e, x, y, z, r);
 }
 
 __device__ __forceinline__ void xform(const Frame &T, float4 c, float &x, float &y, float &z)

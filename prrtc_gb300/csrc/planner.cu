@@ -231,6 +231,7 @@ extern "C" prrtc_status prrtc_solve(prrtc_ctx *ctx, prrtc_robot robot, const flo
     prrtc_robot_limits(robot, P.scale, P.offset);
     P.env = e->dev;
     P.env_n = e->counts;
+    P.grid = e->grid;
     P.ctl = p->ctl;
     P.path = p->path;
     P.path_cap = p->path_cap;

@@ -16,6 +16,7 @@ struct LaunchEnv {
     EnvCounts counts;
     int sms;             // SM count of the device
     unsigned long long *work;   // [2]: FLOPs, configurations (device, accumulated)
+    const EnvGrid *grid = nullptr;   // the environment's clearance grid (device), or none
 };
 
 // Device control block of one query (replaces the reference's file-scope
@@ -52,6 +53,7 @@ struct PlainParams {
     float scale[16], offset[16];       // joint scaling (Robots.hh scale_cfg)
     const float4 *env;
     EnvCounts env_n;
+    const EnvGrid *grid;
     QueryCtl *ctl;
     float *path;                       // [2][path_cap][dof]
     int path_cap;
@@ -64,6 +66,8 @@ struct BatchQueryDesc {
     EnvCounts env_n;
     int cfg_off;         // float offset of start (dof floats) then goals in the config pool
     int num_goals;
+    const EnvGrid *grid; // clearance grid (device), or none
+    int build;           // 1: the batch builds the grid (an uploaded environment brings its own)
 };
 
 enum SlotStateCode { SLOT_FREE = 0, SLOT_RUNNING = 1, SLOT_DONE = 2, SLOT_BUSY = 3 };
@@ -200,6 +204,12 @@ struct GoalQuery {
     float lo[3], hi[3];
     float scale[16], offset[16];  // the robot's joint box
 };
+
+// Clearance grids (env_grid.cu): device bytes of one with at most `cells`
+// cells (a multiple of 16), and the launch that builds those of the n
+// descriptors that ask for it (device array `many`, or the single `one`).
+size_t env_grid_bytes(int cells);
+cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st);
 
 struct ClrLaunch;   // clearance_device.cuh
 struct Ctx;         // context.h

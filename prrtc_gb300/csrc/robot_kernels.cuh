@@ -50,14 +50,16 @@ struct ValidateLaunch {
 
 template <class Gen>
 __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaunch<Gen>::kMinBlocks)
-    k_validate_configs(const float4 *__restrict__ env, EnvCounts nc,
+    k_validate_configs(const float4 *__restrict__ env, EnvCounts nc, const EnvGrid *grid,
                                                           const float *__restrict__ q, int64_t n,
                                                           uint8_t *__restrict__ out, unsigned long long *work)
 {
     extern __shared__ float4 s_env[];
     __shared__ unsigned long long s_bar;
-    stage_env_bulk(s_env, env, nc.records(), &s_bar);
-    CheckCtx ctx{{s_env, nc}, 0.0f, nullptr};
+    __shared__ EnvGrid s_grid;
+    const EnvGrid *gr = stage_grid(&s_grid, grid);
+    stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
+    CheckCtx ctx{{s_env, nc, gr}, 0.0f, nullptr};
     unsigned long long flops = 0, cfgs = 0;
     // The warp steps through the grid-stride loop together (a warp-uniform
     // trip count) and meets at __syncwarp after every configuration: lanes
@@ -88,6 +90,7 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
 // 32-thread blocks of short edges, which keep the unconstrained build (0).
 template <class Gen, int MinBlocks>
 __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
+                                                        const EnvGrid *grid,
                                                         const float *__restrict__ a, const float *__restrict__ b,
                                                         int64_t n, int g, uint8_t *__restrict__ out,
                                                         unsigned long long *work)
@@ -98,8 +101,10 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
     __shared__ float s_a[D], s_step[D];
     __shared__ int s_bad;
     __shared__ unsigned long long s_bar;
-    stage_env_bulk(s_env, env, nc.records(), &s_bar);
-    CheckCtx ctx{{s_env, nc}, 0.0f, &s_bad};
+    __shared__ EnvGrid s_grid;
+    const EnvGrid *gr = stage_grid(&s_grid, grid);
+    stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
+    CheckCtx ctx{{s_env, nc, gr}, 0.0f, &s_bad};
     const float fg = (float)g;
     for (int64_t e = blockIdx.x; e < n; e += gridDim.x) {
         __syncthreads();
@@ -129,13 +134,15 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
 // Goal-region candidates: flags[t] = 1 when candidate t (goal_candidate)
 // puts the chosen sphere's centre in the box and the checker finds it free.
 template <class Gen>
-__global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ env, EnvCounts nc, const GoalQuery g,
-                                                    uint8_t *__restrict__ flags)
+__global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ env, EnvCounts nc,
+                                                    const EnvGrid *grid, const GoalQuery g, uint8_t *__restrict__ flags)
 {
     extern __shared__ float4 s_env[];
     __shared__ unsigned long long s_bar;
-    stage_env_bulk(s_env, env, nc.records(), &s_bar);
-    CheckCtx ctx{{s_env, nc}, 0.0f, nullptr};
+    __shared__ EnvGrid s_grid;
+    const EnvGrid *gr = stage_grid(&s_grid, grid);
+    stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
+    CheckCtx ctx{{s_env, nc, gr}, 0.0f, nullptr};
     // warp-uniform trip count, lanes meeting after every candidate (as in k_validate_configs)
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long tw = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); tw < g.tries; tw += stride) {
@@ -210,8 +217,10 @@ __global__ void __launch_bounds__(256) k_rrtc_plain(const PlainParams P)
         s_hn[tid] = 0.0f;
         s_hd[tid] = 1.0f;
     }
+    __shared__ EnvGrid s_grid;
+    const EnvGrid *gr = stage_grid(&s_grid, P.grid);
     stage_env_bulk(s_env, P.env, P.env_n.records(), &s_bar);   // synchronises the block
-    CheckCtx ctx{{s_env, P.env_n}, P.pad, &s_bad};
+    CheckCtx ctx{{s_env, P.env_n, gr}, P.pad, &s_bad};
     const float fg = (float)P.granularity;
     const unsigned long long t0 = P.budget_ns ? global_ns() : 0ull;
     int iter = 0;
@@ -409,7 +418,7 @@ struct RobotKernels {
         if (n <= 0) return cudaSuccess;
         const int threads = 128;
         const size_t smem = (size_t)le.counts.records() * sizeof(float4);
-        k_validate_configs<Gen><<<grid_for(n, threads, le.sms, 16), threads, smem, st>>>(le.rec, le.counts, q, n, out, le.work);
+        k_validate_configs<Gen><<<grid_for(n, threads, le.sms, 16), threads, smem, st>>>(le.rec, le.counts, le.grid, q, n, out, le.work);
         return cudaGetLastError();
     }
     static cudaError_t validate_edges(const LaunchEnv &le, const float *a, const float *b, int64_t n, int g,
@@ -422,9 +431,9 @@ struct RobotKernels {
         const int64_t cap = (int64_t)le.sms * (2048 / threads);
         if (blocks > cap) blocks = cap;
         if (threads == 128)
-            k_validate_edges<Gen, 8><<<(int)blocks, threads, smem, st>>>(le.rec, le.counts, a, b, n, g, out, le.work);
+            k_validate_edges<Gen, 8><<<(int)blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
         else
-            k_validate_edges<Gen, 0><<<(int)blocks, threads, smem, st>>>(le.rec, le.counts, a, b, n, g, out, le.work);
+            k_validate_edges<Gen, 0><<<(int)blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
         return cudaGetLastError();
     }
     static cudaError_t fk_spheres(const float *q, int64_t n, float *out, int sms, cudaStream_t st)
@@ -467,7 +476,7 @@ struct RobotKernels {
     {
         if (g.tries <= 0) return cudaSuccess;
         const size_t smem = (size_t)le.counts.records() * sizeof(float4);
-        k_goal_flags<Gen><<<grid_for(g.tries, 128, le.sms, 16), 128, smem, st>>>(le.rec, le.counts, g, flags);
+        k_goal_flags<Gen><<<grid_for(g.tries, 128, le.sms, 16), 128, smem, st>>>(le.rec, le.counts, le.grid, g, flags);
         return cudaGetLastError();
     }
     static cudaError_t smooth_paths(const ClrLaunch &P, size_t env_bytes, cudaStream_t st)
