@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
     int cq = 0, catt = 0;   // the slot's query and attempt, read when this warp takes the slot
     bool fresh = true;
     bool trapped = false;   // this warp's last round on its slot was rejected early in full
-    unsigned idle = 0;
+    unsigned idle = 0, scan_from = 0;
     const float4 *staged = nullptr;   // the global records now in W_env
     const EnvGrid *staged_grid = nullptr;   // the grid whose header is in W.grid
     const unsigned env_bar = (unsigned)__cvta_generic_to_shared(&W.env_bar);
@@ -592,62 +592,80 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
         // ---- find work: a pending query, else a running attempt with room for
         // another warp; in the tail, free slots become extra attempts
         if (slot < 0) {
+            // The warp looks at 32 slots at a time, in slot order from a shared
+            // cursor.  A warp that found nothing looks on from where it was:
+            // thousands of idle warps polling the cursor held up the working
+            // ones (one query worked by one warp, the others idle: the launch
+            // took 0.31 ms, 64 polls over 0.28 ms).
             int found = -1, admit = -1, rec = -1, free_slot = -1, free_cand = -1, joinable = 0;
-            unsigned s0 = 0;
-            if (lane == 0) {
-                s0 = atomicAdd((unsigned *)&C->cursor, 1u);
-                const bool pending = vload(&C->admit_next) < P.num_queries;
-                const unsigned long long now = global_ns();
-                for (int tries = 0; tries < P.num_slots; tries++) {
-                    const int s = (int)((s0 + (unsigned)tries) % (unsigned)P.num_slots);
-                    SlotState *S = &P.slots[s];
-                    const int st = vload(&S->state);
-                    if (st == SLOT_FREE && pending && s < P.admit_slots) {
-                        if (atomicCAS(&S->state, SLOT_FREE, SLOT_BUSY) != SLOT_FREE) continue;
-                        int qa = atomicAdd(&C->admit_next, 1);
-                        if (qa < P.num_queries) {
-                            if (P.order) qa = P.order[qa];
-                            open_query(P, qa);
+            if (idle == 0) {
+                if (lane == 0) scan_from = atomicAdd((unsigned *)&C->cursor, 1u);
+                scan_from = __shfl_sync(FULL, scan_from, 0);
+            } else {
+                scan_from++;
+            }
+            const unsigned s0 = scan_from;
+            const bool pending = vload(&C->admit_next) < P.num_queries;
+            const unsigned long long now = global_ns();
+            for (int base = 0; base < P.num_slots && found < 0 && rec < 0; base += 32) {
+                const int s = (int)((s0 + (unsigned)(base + lane)) % (unsigned)P.num_slots);
+                const bool have = base + lane < P.num_slots;
+                const int st = have ? vload(&P.slots[s].state) : SLOT_BUSY;
+                bool run = st == SLOT_RUNNING;
+                int w = 0;
+                if (run) {
+                    w = vload(&P.slots[s].workers);
+                    run = w < P.max_workers;
+                }
+                // a young attempt takes few warps: idle warps that all join
+                // it at once (the tail of a stream) see two small trees,
+                // send half their samples to the free one, and its connect
+                // steps fill the arena.  It counts as joinable all the same
+                // (the warp waits for it instead of forcing another attempt).
+                const bool young = run && w >= kJoinBase &&
+                                   now - *(const volatile unsigned long long *)&P.slots[s].t_start < kJoinYoungNs;
+                const unsigned free_m = __ballot_sync(FULL, st == SLOT_FREE);
+                const unsigned admit_m = __ballot_sync(FULL, st == SLOT_FREE && pending && s < P.admit_slots);
+                if (__any_sync(FULL, run)) joinable = 1;
+                if (free_m && free_cand < 0 && P.max_attempts > 1 && !pending)
+                    free_cand = __shfl_sync(FULL, s, __ffs(free_m) - 1);   // claimed below, only if there is nothing to join
+                unsigned m = __ballot_sync(FULL, run && !young) | admit_m;
+                for (; m && found < 0 && rec < 0; m &= m - 1) {
+                    const int j = __ffs(m) - 1, sj = __shfl_sync(FULL, s, j);
+                    int take = 0, qa = -1;   // 1: slot taken, 2: slot to leave again
+                    if (lane == 0) {
+                        SlotState *S = &P.slots[sj];
+                        if (admit_m >> j & 1) {
+                            if (atomicCAS(&S->state, SLOT_FREE, SLOT_BUSY) == SLOT_FREE) {
+                                qa = atomicAdd(&C->admit_next, 1);
+                                if (qa < P.num_queries) {
+                                    if (P.order) qa = P.order[qa];
+                                    open_query(P, qa);
+                                    atomicAdd(&S->workers, 1);
+                                    take = 1;
+                                } else {
+                                    qa = -1;
+                                    atomicExch(&S->state, SLOT_FREE);
+                                }
+                            }
+                        } else if (vload(&S->workers) < P.max_workers) {
                             atomicAdd(&S->workers, 1);
-                            found = s;
-                            admit = qa;
-                            break;
+                            take = vload(&S->state) == SLOT_RUNNING ? 1 : 2;   // 2: leave it again (possibly recycling it)
                         }
-                        atomicExch(&S->state, SLOT_FREE);
-                    } else if (st == SLOT_FREE && free_cand < 0 && P.max_attempts > 1 && !pending) {
-                        free_cand = s;   // claimed below, only if there is nothing to join
-                    } else if (st == SLOT_RUNNING) {
-                        const int w = vload(&S->workers);
-                        if (w >= P.max_workers) continue;
-                        // a young attempt takes few warps: idle warps that all join
-                        // it at once (the tail of a stream) see two small trees,
-                        // send half their samples to the free one, and its connect
-                        // steps fill the arena.  It counts as joinable all the same
-                        // (the warp waits for it instead of forcing another attempt).
-                        if (w >= kJoinBase &&
-                            now - *(const volatile unsigned long long *)&S->t_start < kJoinYoungNs) {
-                            joinable = 1;
-                            continue;
-                        }
-                        joinable = 1;
-                        atomicAdd(&S->workers, 1);
-                        if (vload(&S->state) == SLOT_RUNNING)
-                            found = s;
-                        else
-                            rec = s;        // leave it again (possibly recycling it)
-                        break;
+                    }
+                    take = __shfl_sync(FULL, take, 0);
+                    if (take == 1) {
+                        found = sj;
+                        admit = __shfl_sync(FULL, qa, 0);
+                    } else if (take == 2) {
+                        rec = sj;
                     }
                 }
-                if (free_cand >= 0 && found < 0 && rec < 0 &&
-                    atomicCAS(&P.slots[free_cand].state, SLOT_FREE, SLOT_BUSY) == SLOT_FREE)
-                    free_slot = free_cand;
             }
-            found = __shfl_sync(FULL, found, 0);
-            admit = __shfl_sync(FULL, admit, 0);
-            rec = __shfl_sync(FULL, rec, 0);
-            free_slot = __shfl_sync(FULL, free_slot, 0);
-            joinable = __shfl_sync(FULL, joinable, 0);
-            s0 = __shfl_sync(FULL, s0, 0);
+            if (free_cand >= 0 && found < 0 && rec < 0) {
+                if (lane == 0 && atomicCAS(&P.slots[free_cand].state, SLOT_FREE, SLOT_BUSY) == SLOT_FREE) free_slot = free_cand;
+                free_slot = __shfl_sync(FULL, free_slot, 0);
+            }
             if (free_slot >= 0) {
                 // nothing to join: an extra attempt of a running query
                 const int qc = spawn_candidate(P, s0 * 7919u, global_ns(), !joinable);
