@@ -780,9 +780,7 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
         }
         if (Qd.grid && staged_grid != Qd.grid) {
             __syncwarp();
-            constexpr int words = sizeof(EnvGrid) / sizeof(int);
-            for (int i = lane; i < words; i += 32)
-                reinterpret_cast<int *>(&W.grid)[i] = __ldg(reinterpret_cast<const int *>(Qd.grid) + i);
+            stage_grid(&W.grid, Qd.grid, envp, lane, 32);
             __syncwarp();
             staged_grid = Qd.grid;
         }

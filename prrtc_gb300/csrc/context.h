@@ -73,6 +73,8 @@ struct Ctx {
     float *bases = nullptr;                 // Halton prime bases per sampling lane [lanes][16]
     int bases_lanes = 0;
     struct Arena *arena = nullptr;          // batched-planner arena kept between batches
+    Buf grids;                              // clearance grids' memory kept between batches (at most kGridsKept)
+    bool grids_in_use = false;              // by a live batch
     unsigned long long *work_dev = nullptr; // [2] FLOPs, configurations (prrtc_work_counters)
     float plan_pad = 0.0f;                  // prrtc_set_planning_margin
     unsigned long long budget_ns = 0;       // prrtc_set_time_budget

@@ -3,6 +3,7 @@
 // routines the generated checkers call for leaf spheres.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -42,11 +43,14 @@ struct EnvCounts {
 // rounded down, 255 for "at least that far".  They bound the reference's
 // tests themselves (env_grid.cu says how), so skipping an obstacle never
 // changes a verdict.
-struct EnvGrid {
+struct alignas(16) EnvGrid {
     float inv[3], off[3];   // a point's cell along an axis: round(p * inv + off)
     int n[3];               // cells per axis, x fastest; 0: the environment has no grid cells
     int cost;               // FLOPs of a sphere tested against every obstacle
+    float out_r;            // a sphere smaller than this centred outside the cells hits nothing
     float lo[3], hi[3];     // box around the obstacles; lo > hi: the grid is not to be used
+    EnvCounts counts;
+    const float4 *rec;      // the obstacles (a staged copy of the header: the staged records, if any)
     const uint8_t *near_;   // per cell: bound of the nearest obstacle
     const uint4 *list;      // per cell two uint4: 16 bounds (15 obstacles, by number; then the next one's), 16 numbers
 };
@@ -119,14 +123,17 @@ __device__ __forceinline__ void stage_env_bulk(float4 *smem, const float4 *__res
     }
 }
 
-// Copy a grid's header into shared memory (all threads of the block
-// participate; caller synchronises); returns the copy, or null for none.
-__device__ __forceinline__ const EnvGrid *stage_grid(EnvGrid *smem, const EnvGrid *__restrict__ g)
+// Copy a grid's header into shared memory (threads t = 0 .. of `stride`
+// participate; caller synchronises), with rec, where its obstacles are staged,
+// in the place of the header's own; returns the copy, or null for none.
+__device__ __forceinline__ const EnvGrid *stage_grid(EnvGrid *smem, const EnvGrid *__restrict__ g, const float4 *rec,
+                                                     int t, int stride)
 {
-    constexpr int words = sizeof(EnvGrid) / sizeof(int);
+    constexpr int words = sizeof(EnvGrid) / sizeof(int), at = offsetof(EnvGrid, rec) / sizeof(int);
     if (!g) return nullptr;
-    for (int i = threadIdx.x; i < words; i += blockDim.x)
-        reinterpret_cast<int *>(smem)[i] = __ldg(reinterpret_cast<const int *>(g) + i);
+    for (int i = t; i < words; i += stride)
+        if (i < at || i >= at + 2) reinterpret_cast<int *>(smem)[i] = __ldg(reinterpret_cast<const int *>(g) + i);
+    if (t == 0) smem->rec = rec;
     return smem;
 }
 
@@ -256,11 +263,18 @@ __device__ __forceinline__ int env_cost(const EnvCounts &n, int k)
 }
 
 // Sphere against obstacle k: 0 no hit, 1 hit, 2 too near contact to tell
-// here.  The distance is the reference test's; what is left to env_hit_all is
-// a band around contact wider than any rounding (coordinates are at most
-// kGridReach, so a distance's rounding is near 1e-5 m at most), so that
-// verdicts do not depend on how two copies of a formula are contracted.
-constexpr float kGridReach = 16.0f;
+// here.  The distance is the reference test's; what is left to the exact test
+// is a band of +-6e-6 m around contact, wider than any rounding (coordinates
+// are at most kGridReach, so a distance's own rounding is below 4e-6 m, and two
+// forms of the kinematics differ by less than 1e-6 m), so that verdicts do
+// not depend on how two copies of a formula are contracted.
+constexpr float kGridReach = 8.0f;
+__device__ __forceinline__ int near_verdict(float d2, float rs)
+{
+    const float s2 = rs * rs, v = d2 - s2, band = 1e-6f * (d2 + s2) + 1.2e-5f * fabsf(rs);
+    return v > band ? 0 : v < -band ? 1 : 2;   // NaN: 2
+}
+
 __device__ __forceinline__ int near_test(const float4 *__restrict__ rec, const EnvCounts &n, int k, float x, float y,
                                          float z, float r)
 {
@@ -293,8 +307,7 @@ __device__ __forceinline__ int near_test(const float4 *__restrict__ rec, const E
         d2 = a1 * a1 + a2 * a2 + a3 * a3;
         rs = r;
     }
-    const float v = d2 - rs * rs, band = 1e-5f * (d2 + rs * rs) + 4e-5f * fabsf(rs);
-    return v > band ? 0 : v < -band ? 1 : 2;
+    return near_verdict(d2, rs);
 }
 
 // the cell of a point, -1 outside the cells (any NaN coordinate, too).  The
@@ -310,10 +323,29 @@ __device__ __forceinline__ int grid_cell(const EnvGrid &g, float x, float y, flo
     return in ? (int)(ix + g.n[0] * (iy + g.n[1] * iz)) : -1;
 }
 
+// A sphere centred outside the cells, by the box around the obstacles: true
+// when it cannot hit any (finite coordinates only).
+__device__ __forceinline__ bool outside(const EnvGrid &g, float x, float y, float z, float ra)
+{
+    const float dx = fmaxf(fmaxf(g.lo[0] - x, x - g.hi[0]), 0.0f), dy = fmaxf(fmaxf(g.lo[1] - y, y - g.hi[1]), 0.0f),
+                dz = fmaxf(fmaxf(g.lo[2] - z, z - g.hi[2]), 0.0f);
+    const float rs = ra * 1.01f + 1e-3f;
+    return g.lo[0] <= g.hi[0] && fabsf(x) + fabsf(y) + fabsf(z) < 1e4f && dx * dx + dy * dy + dz * dz > rs * rs;
+}
+
 // one bit per byte of w that is below t (both unsigned, t <= 255)
 __device__ __forceinline__ unsigned bytes_below(unsigned w, unsigned t4)
 {
-    return ((__vcmpltu4(w, t4) & 0x01010101u) * 0x01020408u) >> 24;
+    return ((__vcmpltu4(w, t4) & 0x01010101u) * 0x01020408u) >> 24 & 15u;
+}
+
+// the listed obstacles of a cell nearer than t (grid units, at most 255), one
+// bit per entry; bit kGridListed: there may be more than those listed
+__device__ __forceinline__ unsigned listed_below(const EnvGrid &g, int cell, int t)
+{
+    const uint4 lb = __ldg(g.list + 2 * cell);
+    const unsigned t4 = (unsigned)t * 0x01010101u;
+    return bytes_below(lb.x, t4) | bytes_below(lb.y, t4) << 4 | bytes_below(lb.z, t4) << 8 | bytes_below(lb.w, t4) << 12;
 }
 
 // Sphere against every obstacle by the clearance grid, result as env_hit's;
@@ -325,22 +357,11 @@ __device__ __forceinline__ int grid_hit(const EnvView &e, float x, float y, floa
     const float ra = fabsf(r);
     const int none = 2 * g.cost;
     const int cell = grid_cell(g, x, y, z);
-    if (cell < 0) {   // outside the cells: by the box around the obstacles (finite coordinates only)
-        const float dx = fmaxf(fmaxf(g.lo[0] - x, x - g.hi[0]), 0.0f), dy = fmaxf(fmaxf(g.lo[1] - y, y - g.hi[1]), 0.0f),
-                    dz = fmaxf(fmaxf(g.lo[2] - z, z - g.hi[2]), 0.0f);
-        const float rs = ra * 1.01f + 1e-3f;
-        const bool sure = g.lo[0] <= g.hi[0] && fabsf(x) + fabsf(y) + fabsf(z) < 1e4f;
-        return sure && dx * dx + dy * dy + dz * dz > rs * rs ? none : -1;
-    }
+    if (cell < 0) return outside(g, x, y, z, ra) ? none : -1;
     const int thr = __float2int_ru(ra * kGridUnit);
     if (thr > 255) return -1;
     if ((int)__ldg(g.near_ + cell) >= thr) return none;
-    const uint4 lb = __ldg(g.list + 2 * cell);
-    const unsigned t4 = (unsigned)thr * 0x01010101u;
-    unsigned m = bytes_below(lb.x, t4) & 15u;
-    m |= (bytes_below(lb.y, t4) & 15u) << 4;
-    m |= (bytes_below(lb.z, t4) & 15u) << 8;
-    m |= (bytes_below(lb.w, t4) & 15u) << 12;
+    unsigned m = listed_below(g, cell, thr);
     if (m >> kGridListed) return -1;
     const uint8_t *num = reinterpret_cast<const uint8_t *>(g.list + 2 * cell + 1);
     while (m) {

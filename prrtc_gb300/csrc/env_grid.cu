@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
     ok = __syncthreads_and(ok);
     if (threadIdx.x == 0) {
         EnvGrid g{};
+        g.out_r = -1.0f;
         float cells[3], from[3], ext[3];
         for (int i = 0; i < 3; i++) {
             for (int w = 1; w < kThreads / 32; w++) {
@@ -162,10 +163,13 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
         g.near_ = reinterpret_cast<const uint8_t *>(Q.grid + 1);
         g.list = reinterpret_cast<const uint4 *>(g.near_ + max_cells);
         g.cost = env_cost(n, no);
+        g.counts = n;
+        g.rec = rec;
         if (ok && ext[0] > 1e-3f && ext[1] > 1e-3f && ext[2] > 1e-3f) {
             // cubic cells, at most max_cells of them
             const float size = cbrtf(ext[0] * ext[1] * ext[2] / (float)max_cells);
             for (int i = 0; i < 3; i++) cells[i] = fmaxf(1.0f, fminf(128.0f, floorf(ext[i] / size)));
+            g.out_r = 0.95f * kInflate;
             while (cells[0] * cells[1] * cells[2] > (float)max_cells) {
                 const int i = cells[0] >= cells[1] && cells[0] >= cells[2] ? 0 : cells[1] >= cells[2] ? 1 : 2;
                 cells[i] -= 1.0f;
@@ -174,6 +178,7 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
                 g.n[i] = (int)cells[i];
                 g.inv[i] = cells[i] / ext[i];
                 g.off[i] = -from[i] * g.inv[i] - 0.5f;
+                if (b.lo[i] - kInflate < -kRoom || b.hi[i] + kInflate > kRoom) g.out_r = -1.0f;
             }
         }
         s_g = g;
@@ -257,6 +262,8 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
 
 }  // namespace
 
+// (the lists, 16-byte entries, follow the header and a multiple of 16 bytes)
+static_assert(sizeof(EnvGrid) % 16 == 0, "the lists behind the header are 16-byte entries");
 size_t env_grid_bytes(int cells) { return sizeof(EnvGrid) + (size_t)cells * 33; }
 
 cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st)

@@ -1,0 +1,217 @@
+// The fast form of the table-driven checkers.
+//
+// Of the tests that the reference's checker makes on a configuration (about
+// 370 sphere-obstacle and 270 sphere-pair tests on the Panda shelf scene)
+// nearly all are far from contact.  The fast form finds those by bounds and
+// makes only the others: straight-line code marks the steps of the schedule
+// whose gate can be hit at all (a byte of the clearance grid per
+// environment gate; one test per pair of frames, then per pair of gates,
+// for self groups), and a walk tests the marked ones in the schedule's
+// order, leaf spheres by the grid's lists and leaf pairs row by row.
+//
+// It answers only where the answer is beyond rounding: a test within 6e-6 m of
+// contact (near_verdict), a configuration out of the range those bounds
+// hold for or an environment without a grid is left to the exact form (about
+// one configuration in a thousand).  So verdicts are the exact form's, bit
+// for bit, and so are the work counts: a test that was skipped counts as the
+// reference makes it.
+#pragma once
+
+#include "device_common.cuh"
+
+namespace prrtc {
+
+enum NearAnswer { kNearHit = 0, kNearFree = 1, kNearUnsure = 2 };
+
+// One step of the schedule for the fast form.
+struct NearStep {
+    int kind;          // 0 environment group, 1 self group
+    int index;
+    short env, self;   // sphere-environment and gate-pair tests of the steps up to and with this one, none hit
+    int tests;         // this step's own sphere-environment tests when nothing hits
+};
+// Leaf pairs of one block (GenPairBlock).  row > 0: rows of `row` pairs with one
+// sphere a each, every row against the same spheres b, all of which lie in
+// the sphere `bound` of frame B.
+struct alignas(16) NearPairBlock {
+    int fa, fb, first, n;
+    float4 bound;
+    int row;
+};
+
+// The environment as the marking code reads it.
+struct NearView {
+    const EnvGrid *g;
+    float pad;
+    int pad_units;   // pad in grid units, rounded up
+};
+
+template <class Ctx>
+__device__ __forceinline__ NearView near_view(const Ctx &ctx)
+{
+    return NearView{ctx.env.grid, ctx.pad, __float2int_ru(ctx.pad * kGridUnit)};
+}
+
+// Can sphere c (radius c.w, `units` in grid units rounded up) touch an obstacle?
+__device__ __forceinline__ bool may_hit_env(const NearView &v, float4 c, int units)
+{
+    const int cell = grid_cell(*v.g, c.x, c.y, c.z);
+    if (cell >= 0) return (int)__ldg(v.g->near_ + cell) < units + v.pad_units;
+    return !(c.w + v.pad < v.g->out_r);
+}
+
+// The same for a sphere larger than the cells' margin around the obstacles:
+// outside the cells by its distance to the box around them.
+__device__ __forceinline__ bool may_hit_env_wide(const NearView &v, float4 c, int units)
+{
+    const int cell = grid_cell(*v.g, c.x, c.y, c.z);
+    return cell >= 0 ? (int)__ldg(v.g->near_ + cell) < units + v.pad_units : !outside(*v.g, c.x, c.y, c.z, c.w + v.pad);
+}
+
+// Can the two spheres (gates, or spheres around several gates) overlap?
+__device__ __forceinline__ bool may_hit_pair(const NearView &v, float4 a, float4 b)
+{
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z, rs = (a.w + b.w) + 2.0f * v.pad + 1e-5f;
+    return dx * dx + dy * dy + dz * dz < rs * rs;
+}
+
+// Sphere against every obstacle: kNearFree (cost: every test's FLOPs),
+// kNearHit (cost: those up to the first hit) or kNearUnsure.
+static __device__ __noinline__ int near_env_all(const EnvGrid *g, float x, float y, float z, float r, int *cost)
+{
+    for (int k = 0; k < g->counts.obstacles(); k++) {
+        const int h = near_test(g->rec, g->counts, k, x, y, z, r);
+        if (h == 2) return kNearUnsure;
+        if (h == 1) {
+            *cost = env_cost(g->counts, k + 1);
+            return kNearHit;
+        }
+    }
+    *cost = g->cost;
+    return kNearFree;
+}
+
+__device__ __forceinline__ int near_env(const EnvGrid *g, float x, float y, float z, float r, int &cost)
+{
+    cost = g->cost;
+    const int cell = grid_cell(*g, x, y, z);
+    if (cell < 0 && outside(*g, x, y, z, r)) return kNearFree;
+    const int t = __float2int_ru(r * kGridUnit);
+    if (cell >= 0 && t <= 255) {
+        if ((int)__ldg(g->near_ + cell) >= t) return kNearFree;
+        unsigned m = listed_below(*g, cell, t);
+        if (!(m >> kGridListed)) {
+            const uint8_t *num = reinterpret_cast<const uint8_t *>(g->list + 2 * cell + 1);
+            for (; m; m &= m - 1) {
+                const int k = __ldg(num + __ffs(m) - 1);
+                const int h = near_test(g->rec, g->counts, k, x, y, z, r);
+                if (h == 2) return kNearUnsure;
+                if (h == 1) {
+                    cost = env_cost(g->counts, k + 1);
+                    return kNearHit;
+                }
+            }
+            return kNearFree;
+        }
+    }
+    int c;
+    const int h = near_env_all(g, x, y, z, r, &c);
+    cost = c;
+    return h;
+}
+
+// Leaf pairs of one block; cost as above.
+__device__ __forceinline__ int near_pairs(const Frame &Tab, const LeafPair *__restrict__ pairs, const NearPairBlock &b,
+                                          float pad2, int &cost)
+{
+    const int row = b.row ? b.row : b.n;
+    unsigned rows = 1;
+    if (b.row) {   // rows whose sphere a is clear of all spheres b cannot hit
+        float x, y, z;
+        xform(Tab, b.bound, x, y, z);
+        rows = 0;
+        for (int i = 0, k = b.first; k < b.first + b.n; i++, k += row) {
+            const float4 a = pairs[k].a;
+            const float dx = a.x - x, dy = a.y - y, dz = a.z - z, rs = a.w + b.bound.w + pad2 + 1e-5f;
+            rows |= (dx * dx + dy * dy + dz * dz < rs * rs ? 1u : 0u) << i;
+        }
+    }
+    for (; rows; rows &= rows - 1) {
+        const int first = (__ffs(rows) - 1) * row;
+        for (int i = first; i < first + row; i++) {
+            const LeafPair p = pairs[b.first + i];
+            float x, y, z;
+            xform(Tab, p.b, x, y, z);
+            const float dx = p.a.x - x, dy = p.a.y - y, dz = p.a.z - z;
+            const int h = near_verdict(dx * dx + dy * dy + dz * dz, p.a.w + p.b.w + pad2);
+            if (h == 2) return kNearUnsure;
+            if (h == 1) {
+                cost = kFlopPair * (i + 1);
+                return kNearHit;
+            }
+        }
+    }
+    cost = kFlopPair * b.n;
+    return kNearFree;
+}
+
+// The steps marked in `word` (32 of the schedule's, from `base` on), in
+// order.  The lanes of a warp take the union of their steps together, so that
+// they read the same table entries and run the same code.  F: frame view, G:
+// gate centres.  Returns NearAnswer + 4 * FLOPs: on a collision those of the
+// whole check so far, else those beyond what the same steps cost with nothing hit
+// (negative where a gate was hit early and its leaves cost less).
+// T: the robot's tables.
+template <class T, class Frames>
+__device__ __noinline__ unsigned near_walk(const Frames F, const float4 *__restrict__ G, unsigned word, int base,
+                                           const EnvGrid *g, float pad, int extra)
+{
+    unsigned todo = __reduce_or_sync(__activemask(), word);
+    for (; todo; todo &= todo - 1) {
+        const int s = __ffs(todo) - 1;
+        if (!(word >> s & 1)) continue;
+        const NearStep e = T::steps()[base + s];
+        int h = kNearFree, c;
+        if (e.kind == 0) {
+            const GenEnvGroup gr = T::env_groups()[e.index];
+            bool go = true;
+            if (gr.gate >= 0) {
+                const float4 p = G[gr.gate];
+                const int a = near_env(g, p.x, p.y, p.z, p.w + pad, c);
+                if (a == kNearUnsure) return kNearUnsure;
+                extra += c;
+                go = a == kNearHit;
+            }
+            if (go)
+                for (int k = gr.first_block; k < gr.first_block + gr.nblocks && h == kNearFree; k++) {
+                    const GenLeafBlock b = T::leaf_blocks()[k];
+                    const Frame A = frame_at(F, b.frame + 1);
+                    for (int i = b.first; i < b.first + b.n && h == kNearFree; i++) {
+                        const float4 l = T::leaves()[i];
+                        float x, y, z;
+                        xform(A, l, x, y, z);
+                        h = near_env(g, x, y, z, l.w + pad, c);
+                        extra += c;
+                    }
+                }
+            extra -= g->cost * e.tests;
+        } else {
+            const GenSelfGroup gr = T::self_groups()[e.index];
+            const float4 a = G[gr.ga], b = G[gr.gb];
+            const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+            const int gate = near_verdict(dx * dx + dy * dy + dz * dz, (a.w + b.w) + 2.0f * pad);
+            if (gate == 2) return kNearUnsure;
+            if (gate == 1)
+                for (int k = gr.first_block; k < gr.first_block + gr.nblocks && h == kNearFree; k++) {
+                    const NearPairBlock b = T::pair_blocks()[k];
+                    h = near_pairs(relative_frame(frame_at(F, b.fa + 1), frame_at(F, b.fb + 1)), T::pairs(), b, 2.0f * pad, c);
+                    extra += c;
+                }
+        }
+        if (h == kNearUnsure) return kNearUnsure;
+        if (h == kNearHit) return kNearHit + 4u * (unsigned)(g->cost * e.env + kFlopPair * e.self + extra);
+    }
+    return kNearFree + 4u * (unsigned)extra;
+}
+
+}  // namespace prrtc

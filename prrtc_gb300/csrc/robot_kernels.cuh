@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
     extern __shared__ float4 s_env[];
     __shared__ unsigned long long s_bar;
     __shared__ EnvGrid s_grid;
-    const EnvGrid *gr = stage_grid(&s_grid, grid);
+    const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
     CheckCtx ctx{{s_env, nc, gr}, 0.0f, nullptr};
     unsigned long long flops = 0, cfgs = 0;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
     __shared__ int s_bad;
     __shared__ unsigned long long s_bar;
     __shared__ EnvGrid s_grid;
-    const EnvGrid *gr = stage_grid(&s_grid, grid);
+    const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
     CheckCtx ctx{{s_env, nc, gr}, 0.0f, &s_bad};
     const float fg = (float)g;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ e
     extern __shared__ float4 s_env[];
     __shared__ unsigned long long s_bar;
     __shared__ EnvGrid s_grid;
-    const EnvGrid *gr = stage_grid(&s_grid, grid);
+    const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
     CheckCtx ctx{{s_env, nc, gr}, 0.0f, nullptr};
     // warp-uniform trip count, lanes meeting after every candidate (as in k_validate_configs)
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) k_rrtc_plain(const PlainParams P)
         s_hd[tid] = 1.0f;
     }
     __shared__ EnvGrid s_grid;
-    const EnvGrid *gr = stage_grid(&s_grid, P.grid);
+    const EnvGrid *gr = stage_grid(&s_grid, P.grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, P.env, P.env_n.records(), &s_bar);   // synchronises the block
     CheckCtx ctx{{s_env, P.env_n, gr}, P.pad, &s_bad};
     const float fg = (float)P.granularity;

@@ -28,6 +28,8 @@ from __future__ import annotations
 import json
 from pathlib import Path
 
+import numpy as np
+
 HERE = Path(__file__).resolve().parent
 CSRC = HERE.parent / "csrc" / "robots"
 ROBOTS = ("sphere", "panda", "fetch", "baxter")
@@ -332,6 +334,12 @@ def emit_cuda_checker(m: dict) -> str:
     for g in m["self_groups"]:
         for sidx in g["gate"]:
             gate_ids.setdefault(sidx, len(gate_ids))
+    # for the fast form the leaves of an ungated environment group stand in for its gate
+    near_ids = dict(gate_ids)
+    for g in m["env_groups"]:
+        if g["gate"] < 0:
+            for leaf in g["leaves"]:
+                near_ids.setdefault(leaf, len(near_ids))
     tcode = None
     if table:
         # every frame, in chain order, into F[q + 1]; then the schedule loop
@@ -403,6 +411,8 @@ def emit_cuda_checker(m: dict) -> str:
     w("// a leaf counts only when its group's gate (bounding sphere or bounding pair)")
     w("// is hit; a config is free when no counted leaf is hit.")
     w("#pragma once")
+    if table:
+        w('#include "../near_check.cuh"')
     w("")
     w(f"namespace prrtc {{ namespace gen_{name} {{")
     w("")
@@ -465,26 +475,57 @@ def emit_cuda_checker(m: dict) -> str:
         for fa, fb, pf, n in pblocks or [(-1, -1, 0, 0)]:
             w(f"    {{{fa}, {fb}, {pf}, {n}}},")
         w("};")
+        w("// the same for the fast form (near_check.cuh)")
+        w(f"__device__ const NearStep k{R}NearStep[{len(m['schedule'])}] = {{")
+        ne = ns = 0
+        for kind, gi in m["schedule"]:
+            n = _env_tests(m, gi) if kind == "env" else 0
+            ne, ns = ne + n, ns + (kind != "env")
+            w(f"    {{{0 if kind == 'env' else 1}, {gi}, {ne}, {ns}, {n}}},")
+        w("};")
+        w(f"__device__ const NearPairBlock k{R}NearPair[{max(1, len(pblocks))}] = {{")
+        for fa, fb, pf, n in pblocks or [(-1, -1, 0, 0)]:
+            row, c, r = _rows(pair_rows[pf:pf + n])
+            w(f"    {{{fa}, {fb}, {pf}, {n}, {{{', '.join(_lit(v) for v in [*c, r])}}}, {row}}},")
+        w("};")
+        w(f"struct {R}Near {{")
+        for name, type_, arr in (("steps", "NearStep", "NearStep"), ("env_groups", "GenEnvGroup", "EnvGroup"),
+                                 ("leaf_blocks", "GenLeafBlock", "LeafBlock"), ("leaves", "float4", "Leaf"),
+                                 ("self_groups", "GenSelfGroup", "SelfGroup"), ("pair_blocks", "NearPairBlock", "NearPair"),
+                                 ("pairs", "LeafPair", "Pair")):
+            w(f"    static __device__ __forceinline__ const {type_} *{name}() {{ return k{R}{arr}; }}")
+        w("};")
     w("")
-    w("// Returns true when configuration q is collision-free.")
-    w("template <class Ctx>")
-    w("__device__ __forceinline__ bool fkcc(const float *__restrict__ q, Ctx &ctx)")
-    w("{")
-    for line in (tcode if table else code).lines:
-        w("    " + line)
-    w("}")
-    w("")
-    w("// The same verdicts for the stand-alone checker of single configurations.")
-    w("template <class Ctx>")
-    w("__device__ __forceinline__ bool fkcc_validate(const float *__restrict__ q, Ctx &ctx)")
-    w("{")
-    if table and inline:
-        for line in code.lines:
+
+    def function(head, lines):
+        w("template <class Ctx>")
+        w(f"{head}(const float *__restrict__ q, Ctx &ctx)")
+        w("{")
+        for line in lines:
             w("    " + line)
-    else:
-        w("    return fkcc(q, ctx);")
-    w("}")
-    w("")
+        w("}")
+        w("")
+
+    def fast_or(exact, near):
+        """The fast form's answer, else the exact form's (on values the
+        compiler cannot tell from new ones, so that it keeps none of the fast
+        form's kinematics for them)."""
+        return [f"const int a = {near}(q, ctx);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
+                "#pragma unroll", "for (int d = 0; d < kDof; d++) {", "    c[d] = q[d];",
+                '    asm volatile("" : "+f"(c[d]));', "}", f"return {exact}(c, ctx);"]
+
+    if table:
+        function("__device__ __forceinline__ bool fkcc_exact", tcode.lines)
+        if inline:
+            function("__device__ __forceinline__ bool fkcc_validate_exact", code.lines)
+        function("__device__ __forceinline__ int fkcc_near", _near_body(m, near_ids, store_late=False))
+        if inline:
+            function("__device__ __forceinline__ int fkcc_validate_near", _near_body(m, near_ids, store_late=True))
+    w("// Returns true when configuration q is collision-free.")
+    function("__device__ __forceinline__ bool fkcc", fast_or("fkcc_exact", "fkcc_near") if table else code.lines)
+    w("// The same verdicts for the stand-alone checker of single configurations.")
+    function("__device__ __forceinline__ bool fkcc_validate",
+             fast_or("fkcc_validate_exact", "fkcc_validate_near") if table and inline else ["return fkcc(q, ctx);"])
     w("// World centre and radius of every model sphere (model sphere order).")
     w("__device__ __forceinline__ void fk_spheres(const float *__restrict__ q, float4 *__restrict__ out)")
     w("{")
@@ -495,6 +536,142 @@ def emit_cuda_checker(m: dict) -> str:
     w(f"}} }}  // namespace prrtc::gen_{name}")
     w("")
     return "\n".join(out)
+
+
+def _bounding_sphere(spheres):
+    """(centre, radius) of a sphere around the given (centre, radius) spheres,
+    radius rounded up."""
+    c = np.mean([s[0] for s in spheres], axis=0)
+    for k in range(2000):          # towards the farthest one, by shrinking steps
+        d = [np.linalg.norm(np.asarray(x) - c) + r for x, r in spheres]
+        i = int(np.argmax(d))
+        v = np.asarray(spheres[i][0]) - c
+        n = np.linalg.norm(v)
+        if n < 1e-12:
+            break
+        c = c + v / n * min(n, d[i] * 0.5 / (k + 2))
+    return [float(x) for x in c], float(max(np.linalg.norm(np.asarray(x) - c) + r for x, r in spheres)) + 1e-5
+
+
+GRID_UNIT = 512        # kGridUnit, device_common.cuh
+WIDE = 0.19            # spheres above EnvGrid::out_r (env_grid.cu: 0.95 x 0.2 m)
+CLUSTER = 3            # gate pairs of two frames that are worth a test of the frames' gates as a whole
+
+
+def _near_body(m, gate_ids, store_late):
+    """The fast form (near_check.cuh): frames, gate centres, the marks of the
+    schedule's steps that can hit, then the walk over those.  store_late: the
+    frames and centres that the walk reads are stored only by lanes that walk."""
+    R = m["robot"].capitalize()
+    code = _Code()
+    fk = _FkGen(m, code)
+    sp, nj, w = m["spheres"], len(m["joints"]), code.lines.append
+    w("const EnvGrid *grid = ctx.env.grid;")
+    w("if (!grid || !(grid->lo[0] <= grid->hi[0])) return kNearUnsure;")
+    w(f"if (!({' + '.join(f'fabsf(q[{d}])' for d in range(m['dof']))} < 100.0f)) return kNearUnsure;")
+    for jt in m["joints"]:
+        if jt["type"] != "revolute":
+            w(f"if (fabsf(q[{jt['q']}]) > 4.0f) return kNearUnsure;")
+    frames = [fk.frame(jt["q"]) for jt in m["joints"]]
+    fexpr = {-1: "world_frame()"} | {jt["q"]: _frame_arg(T) for jt, T in zip(m["joints"], frames)}
+    w(f"FrameStore<Ctx, {nj + 1}> F(ctx);")
+    w(f"float4 G[{max(1, len(gate_ids))}];")
+    store = [f"F.set({jt['q'] + 1}, {_frame_arg(T)});" for jt, T in zip(m["joints"], frames)]
+    if not store_late:
+        code.lines += store
+        store = []
+    # gate centres in world coordinates, from the frames still in registers
+    for sidx, gid in gate_ids.items():
+        c = [float(np.float32(v)) for v in (*sp[sidx]["c"], sp[sidx]["r"])]
+        w(f"const float4 g{gid} = gate_centre({fexpr[sp[sidx]['frame']]}, make_float4({', '.join(_lit(v) for v in c)}));")
+        if store_late:
+            store.append(f"G[{gid}] = g{gid};")
+        else:
+            w(f"G[{gid}] = g{gid};")
+    w("const NearView near = near_view(ctx);")
+    steps = m["schedule"]
+    words = (len(steps) + 31) // 32
+    w("unsigned " + ", ".join(f"m{k} = 0" for k in range(words)) + ";")
+
+    def mark(s, cond):
+        return f"m{s >> 5} |= {cond} ? {hex(1 << (s & 31))}u : 0u;"
+
+    pairs = {}
+    for s, (kind, gi) in enumerate(steps):
+        if kind == "env":
+            g = m["env_groups"][gi]
+            for sidx in ([g["gate"]] if g["gate"] >= 0 else g["leaves"]):
+                r = np.float32(sp[sidx]["r"])
+                units = int(np.ceil(float(r) * GRID_UNIT))
+                w(mark(s, f"may_hit_env{'_wide' if r >= WIDE else ''}(near, g{gate_ids[sidx]}, {units})"))
+        else:
+            a, b = m["self_groups"][gi]["gate"]
+            key = tuple(sp[x]["frame"] if sp[x]["frame"] >= 0 else ("world", x) for x in (a, b))
+            pairs.setdefault(key, []).append((s, a, b))
+    clusters = {}
+
+    def cluster(key, gates):
+        """The centre of the sphere around a frame's gates, emitted once."""
+        if not isinstance(key, int) or len(gates) == 1:
+            return f"g{gate_ids[gates[0]]}"
+        name = f"b{key}_" + "_".join(str(gate_ids[x]) for x in gates)
+        if name not in clusters:
+            c, r = _bounding_sphere([(np.float32(sp[x]["c"]).astype(float), float(np.float32(sp[x]["r"]))) for x in gates])
+            clusters[name] = f"c{key}_{len(clusters)}"
+            w(f"const float4 {clusters[name]} = gate_centre({fexpr[key]}, make_float4({', '.join(_lit(v) for v in [*c, r])}));")
+        return clusters[name]
+
+    for (ka, kb), list_ in pairs.items():
+        test = [mark(s, f"may_hit_pair(near, g{gate_ids[a]}, g{gate_ids[b]})") for s, a, b in list_]
+        if len(list_) >= CLUSTER:
+            ca = cluster(ka, sorted({a for _, a, _ in list_}))
+            cb = cluster(kb, sorted({b for _, _, b in list_}))
+            w(f"if (may_hit_pair(near, {ca}, {cb})) {{")
+            code.lines += ["    " + t for t in test]
+            w("}")
+        else:
+            code.lines += test
+    any_ = " | ".join(f"m{k}" for k in range(words))
+    env_total = sum(_env_tests(m, gi) for kind, gi in steps if kind == "env")
+    self_total = sum(kind != "env" for kind, _ in steps)
+    w("int extra = 0;")
+    w(f"if ({any_}) {{")
+    w("    if (ctx.stop()) return kNearFree;")
+    code.lines += ["    " + t for t in store]
+    for k in range(words):
+        w(f"    if (m{k}) {{")
+        w(f"        const unsigned a = near_walk<{R}Near>(F.view(), G, m{k}, {32 * k}, grid, ctx.pad, extra);")
+        w("        if ((a & 3u) == kNearHit) ctx.work += a >> 2;")
+        w("        if ((a & 3u) != kNearFree) return (int)(a & 3u);")
+        w("        extra = (int)a >> 2;")
+        w("    }")
+    w("}")
+    w(f"ctx.work += (unsigned)(grid->cost * {env_total} + kFlopPair * {self_total} + extra);")
+    w("return kNearFree;")
+    return code.lines
+
+
+def _rows(rows):
+    """(row, centre, radius) of a block of pairs (ca, ra, cb, rb): `row` pairs
+    per sphere a, every a against the same spheres b, which the sphere
+    (centre, radius) encloses; row = 0 where the block is not of that form or
+    skipping rows saves nothing."""
+    f = lambda v: [float(np.float32(x)) for x in v]  # noqa: E731
+    a = [(tuple(r[0]), r[1]) for r in rows]
+    b = [(tuple(r[2]), r[3]) for r in rows]
+    row = next((k for k in range(1, len(a)) if a[k] != a[0]), len(a))
+    if row < 3 or len(a) % row or len(a) // row > 32 or any(
+            a[k] != a[k - k % row] or b[k] != b[k % row] for k in range(len(a))):
+        return 0, [0.0, 0.0, 0.0], 0.0
+    c, r = _bounding_sphere([(np.array(f(x)), float(np.float32(y))) for x, y in b[:row]])
+    c = f(c)   # as the table holds it
+    return row, c, max(float(np.linalg.norm(np.array(f(x)) - np.array(c))) + float(np.float32(y)) for x, y in b[:row]) + 1e-5
+
+
+def _env_tests(m, gi):
+    """Spheres of an environment group tested when nothing hits."""
+    g = m["env_groups"][gi]
+    return 1 if g["gate"] >= 0 else len(g["leaves"])
 
 
 def _op(v):

@@ -44,7 +44,7 @@ def _env(kind):
         return Environment(spheres=spheres(40, (0.45, -0.05, 0.5), (0.55, 0.05, 0.6)),
                            capsules=[capsule_row((0.4, y, 0.3), (0.4, y, 0.7), 0.01) for y in np.linspace(-0.1, 0.1, 20)])
     if kind == "wide floor and walls":
-        return Environment(cuboids=[cuboid_row((0, 0, -0.1), (10, 10, 0.05)), cuboid_row((0.8, 0, 1), (0.02, 10, 2))],
+        return Environment(cuboids=[cuboid_row((0, 0, -0.1), (7, 7, 0.05)), cuboid_row((0.8, 0, 1), (0.02, 7, 2))],
                            spheres=spheres(5))
     if kind == "out of reach":
         return Environment(spheres=[[5.0, 5.0, 5.0, 0.3]], cuboids=[cuboid_row((-8.0, 0.0, 0.0), (0.5, 0.5, 0.5))])
