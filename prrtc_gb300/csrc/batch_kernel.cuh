@@ -56,6 +56,7 @@ struct alignas(16) WarpScratch {
     float pend_d[32];
     unsigned long long env_bar;   // mbarrier of the bulk copies that stage the obstacle records
     EnvGrid grid;                 // the header of the query's clearance grid
+    EnvView view;                 // the query's environment
     int bad;
 };
 
@@ -207,17 +208,30 @@ __device__ __forceinline__ bool sample_group(const BatchParams &P, const WarpScr
     return false;
 }
 
+template <class Ctx>
+__device__ __forceinline__ Ctx make_ctx(const EnvView &view, float pad, volatile int *stop, float4 *frames)
+{
+    if constexpr (Ctx::kSharedFrames)
+        return Ctx{CheckCtx{view, pad, stop}, frames};
+    else
+        return Ctx{view, pad, stop};
+}
+
 // Whole warp: check the g points of the edge in W (from + k * step),
 // k = 1..g, in ceil(g / 32) rounds of one point per lane.  Contiguous order
 // gives round r the points 32 r + lane + 1; interleaved order gives it
 // lane * R + r + 1, so the first round already samples the whole edge at
-// stride R.  Adds the work done to work[0] (FLOPs) and work[1] (points).
+// stride R.  Adds the work done to work[0] (FLOPs) and work[1] (points).  A
+// called function: inlined where edges are extended and connected, with both
+// kinds of frame storage, the checker took the kernel's four copies of it to
+// 168 registers (12 warps per SM).
 template <class Gen, class Ctx>
-__device__ __forceinline__ bool warp_validate(const WarpScratch<Gen::kDof> &W, int g, int interleave, Ctx &ctx,
-                                              unsigned long long *work)
+__device__ __noinline__ bool warp_validate(WarpScratch<Gen::kDof> &W, float4 *frames, int g, int interleave, float pad,
+                                           unsigned long long *work)
 {
     constexpr int D = Gen::kDof;
     const int lane = lane_id();
+    Ctx ctx = make_ctx<Ctx>(W.view, pad, &W.bad, frames);
     volatile int *flag = ctx.stop_flag;
     if (lane == 0) *flag = 0;
     __syncwarp();
@@ -535,8 +549,11 @@ __device__ __forceinline__ int spawn_candidate(const BatchParams &P, unsigned fr
     return -1;
 }
 
+// (at most 168 registers: with 96, 20 instead of 12 warps per SM, the checker's
+// spills cost more than the warps gained: 1024 tabletop queries 4.26 against
+// 3.82 ms a call, 4096 shelf queries 125 against 116 ms)
 template <class Gen>
-__global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
+__global__ void __launch_bounds__(128, 3) k_rrtc_batch(const BatchParams P)
 {
     constexpr int D = Gen::kDof;
     constexpr unsigned FULL = 0xffffffffu;
@@ -729,6 +746,7 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
         // The slot's query and attempt stay fixed while this warp works on it (a
         // slot is reused only after its last worker has left).
         SlotState *S = &P.slots[slot];
+        const bool new_query = fresh;
         if (fresh) {
             if (lane == 0) {
                 cq = vload(&S->query);
@@ -784,12 +802,15 @@ __global__ void __launch_bounds__(128) k_rrtc_batch(const BatchParams P)
             __syncwarp();
             staged_grid = Qd.grid;
         }
-        CheckCtx ctx{{envp, Qd.env_n, Qd.grid ? &W.grid : nullptr}, P.pad, &W.bad};
-        SharedCheckCtx sctx{ctx, W_frames + lane};
+        if (new_query) {
+            if (lane == 0) W.view = EnvView{envp, Qd.env_n, Qd.grid ? &W.grid : nullptr};
+            __syncwarp();
+        }
         // every point of an edge through the robot's checker, frames where P says
         auto validate = [&]() {
-            return P.shared_frames ? warp_validate<Gen>(W, P.granularity, P.edge_order, sctx, C->work)
-                                   : warp_validate<Gen>(W, P.granularity, P.edge_order, ctx, C->work);
+            return P.shared_frames
+                       ? warp_validate<Gen, SharedCheckCtx>(W, W_frames + lane, P.granularity, P.edge_order, P.pad, C->work)
+                       : warp_validate<Gen, CheckCtx>(W, nullptr, P.granularity, P.edge_order, P.pad, C->work);
         };
         float *nodes_s = P.nodes + (size_t)slot * 2 * D * P.cap;
         int *par_s = P.parents + (size_t)slot * 2 * P.cap;

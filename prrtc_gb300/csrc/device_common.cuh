@@ -264,21 +264,21 @@ __device__ __forceinline__ int env_cost(const EnvCounts &n, int k)
 
 // Sphere against obstacle k: 0 no hit, 1 hit, 2 too near contact to tell
 // here.  The distance is the reference test's; what is left to the exact test
-// is a band of +-6e-6 m around contact, wider than any rounding (coordinates
-// are at most kGridReach, so a distance's own rounding is below 4e-6 m, and two
-// forms of the kinematics differ by less than 1e-6 m), so that verdicts do
-// not depend on how two copies of a formula are contracted.
+// is a band around contact wider than any rounding: 2e-6 m (two forms of the
+// kinematics differ by less than 1e-6 m, and so do the distances of spheres
+// that near), and for capsules and boxes 5e-7 of the offset from the
+// obstacle's origin, whose products round by as much.  So verdicts do not
+// depend on how two copies of a formula are contracted.
 constexpr float kGridReach = 8.0f;
-__device__ __forceinline__ int near_verdict(float d2, float rs)
+__device__ __forceinline__ int near_verdict(float d2, float rs, float band = 2e-6f)
 {
-    const float s2 = rs * rs, v = d2 - s2, band = 1e-6f * (d2 + s2) + 1.2e-5f * fabsf(rs);
-    return v > band ? 0 : v < -band ? 1 : 2;   // NaN: 2
+    const float v = d2 - rs * rs, w = 2.0f * band * (fabsf(rs) + band) + 4e-7f * d2;
+    return v > w ? 0 : v < -w ? 1 : 2;   // NaN: 2
 }
-
 __device__ __forceinline__ int near_test(const float4 *__restrict__ rec, const EnvCounts &n, int k, float x, float y,
                                          float z, float r)
 {
-    float d2, rs;
+    float d2, rs, band = 2e-6f;
     if (k < n.ns) {
         const float4 s = rec[k];
         const float dx = x - s.x, dy = y - s.y, dz = z - s.z;
@@ -295,6 +295,7 @@ __device__ __forceinline__ int near_test(const float4 *__restrict__ rec, const E
         const float dx = x - (a.x + v.x * t), dy = y - (a.y + v.y * t), dz = z - (a.z + v.z * t);
         d2 = dx * dx + dy * dy + dz * dz;
         rs = r + a.w;
+        band += 5e-7f * (fabsf(x - a.x) + fabsf(y - a.y) + fabsf(z - a.z));
     } else {
         const bool upright = k >= n.ns + n.nc + n.nzc + n.ncb;
         const float4 *c = rec + n.ns + 2 * (n.nc + n.nzc) + 4 * (k - n.ns - n.nc - n.nzc);
@@ -306,8 +307,9 @@ __device__ __forceinline__ int near_test(const float4 *__restrict__ rec, const E
         const float a3 = fmaxf(0.0f, fabsf(upright ? zs : c3.x * xs + c3.y * ys + c3.z * zs) - c2.w);
         d2 = a1 * a1 + a2 * a2 + a3 * a3;
         rs = r;
+        band += 5e-7f * (fabsf(xs) + fabsf(ys) + fabsf(zs));
     }
-    return near_verdict(d2, rs);
+    return near_verdict(d2, rs, band);
 }
 
 // the cell of a point, -1 outside the cells (any NaN coordinate, too).  The
@@ -532,6 +534,8 @@ __device__ __forceinline__ Frame frame_at(const SharedFrames F, int i)
 // algorithmic FLOPs of the primitive tests executed (reference weights).
 struct CheckCtx {
     static constexpr bool kSharedFrames = false;   // table-form frames in a local array
+    static constexpr bool kInlineExact = false;    // the exact form (near_check.cuh) as a called function
+    static constexpr bool kLeafMarks = true;       // the fast form marks by leaves too (points of one edge)
     EnvView env;
     float pad;
     volatile int *stop_flag;
@@ -560,6 +564,21 @@ struct CheckCtx {
         return dx * dx + dy * dy + dz * dz - rs * rs < 0.0f;
     }
     __device__ __forceinline__ bool stop() const { return stop_flag != nullptr && *stop_flag != 0; }
+};
+
+// The stand-alone configuration checker's: its exact form is compiled into the
+// kernel.  (How a compiler contracts the kinematics' products depends on the
+// code around them; a called copy's verdicts differed from the inlined form's
+// for Panda and Baxter within 1e-8 m of contact, while an edge's points gave
+// the same verdicts either way: 70 M configurations bisected onto contact.)
+struct SingleCheckCtx : CheckCtx {
+    static constexpr bool kInlineExact = true;
+};
+// The same for warps full of unrelated configurations: some lane's gates
+// overlap in nearly every self group, so all the leaf marks' code would run
+// (2^20 random Panda shelf configurations: 1.07 ms with it, 0.83 without).
+struct MixedCheckCtx : SingleCheckCtx {
+    static constexpr bool kLeafMarks = false;
 };
 
 // The same checks with the table-form frames in the warp's shared-memory

@@ -9,7 +9,12 @@
 // for self groups), and a walk tests the marked ones in the schedule's
 // order, leaf spheres by the grid's lists and leaf pairs row by row.
 //
-// It answers only where the answer is beyond rounding: a test within 6e-6 m of
+// The marking code keeps everything in registers (frames die as the chain goes
+// on); a lane with marked steps computes its frames again, into local memory,
+// for the walk (near_resolve): most warps of an edge's points have none, and
+// storing 7 frames and 11 centres for every point had cost more than that.
+//
+// It answers only where the answer is beyond rounding: a test within microns of
 // contact (near_verdict), a configuration out of the range those bounds
 // hold for or an environment without a grid is left to the exact form (about
 // one configuration in a thousand).  So verdicts are the exact form's, bit
@@ -28,7 +33,7 @@ struct NearStep {
     int kind;          // 0 environment group, 1 self group
     int index;
     short env, self;   // sphere-environment and gate-pair tests of the steps up to and with this one, none hit
-    int tests;         // this step's own sphere-environment tests when nothing hits
+    int tests;         // environment: sphere tests of this step when nothing hits; self: its leaf pairs
 };
 // Leaf pairs of one block (GenPairBlock).  row > 0: rows of `row` pairs with one
 // sphere a each, every row against the same spheres b, all of which lie in
@@ -44,12 +49,14 @@ struct NearView {
     const EnvGrid *g;
     float pad;
     int pad_units;   // pad in grid units, rounded up
+    bool wide;       // the pad is more than the leaf marks allow for (kNearPad): gates alone decide
 };
+constexpr float kNearPad = 1e-4f;
 
 template <class Ctx>
 __device__ __forceinline__ NearView near_view(const Ctx &ctx)
 {
-    return NearView{ctx.env.grid, ctx.pad, __float2int_ru(ctx.pad * kGridUnit)};
+    return NearView{ctx.env.grid, ctx.pad, __float2int_ru(ctx.pad * kGridUnit), ctx.pad > kNearPad};
 }
 
 // Can sphere c (radius c.w, `units` in grid units rounded up) touch an obstacle?
@@ -73,6 +80,33 @@ __device__ __forceinline__ bool may_hit_pair(const NearView &v, float4 a, float4
 {
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z, rs = (a.w + b.w) + 2.0f * v.pad + 1e-5f;
     return dx * dx + dy * dy + dz * dz < rs * rs;
+}
+
+// The gate pair's own test (near_verdict).
+__device__ __forceinline__ int near_gate(const NearView &v, float4 a, float4 b)
+{
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    return near_verdict(dx * dx + dy * dy + dz * dz, (a.w + b.w) + 2.0f * v.pad);
+}
+
+// Leaf marks.  A self group whose gates overlap often without its leaves being
+// near (two neighbouring links' gates always do) is marked by its leaves:
+// balls around one link's leaves are brought into the other link's frame
+// (local_point: coordinates and squared length), where that link's leaves are
+// constants, and |a - p|^2 < s^2 is three multiply-adds with immediate operands
+// and a comparison: (-2 a) . p + |p|^2 < s^2 - |a|^2.  A step that its leaves
+// leave unmarked although its gates overlap is `passed`: the reference tests
+// all its leaf pairs, and they count.
+__device__ __forceinline__ float4 local_point(const Frame &T, float4 c)
+{
+    const float dx = c.x - T.m[3], dy = c.y - T.m[7], dz = c.z - T.m[11];
+    const float x = T.m[0] * dx + T.m[4] * dy + T.m[8] * dz, y = T.m[1] * dx + T.m[5] * dy + T.m[9] * dz,
+                z = T.m[2] * dx + T.m[6] * dy + T.m[10] * dz;
+    return make_float4(x, y, z, x * x + y * y + z * z);
+}
+__device__ __forceinline__ bool near_leaf(float4 p, float ax, float ay, float az, float limit)
+{
+    return fmaf(p.x, ax, fmaf(p.y, ay, fmaf(p.z, az, p.w))) < limit;
 }
 
 // Sphere against every obstacle: kNearFree (cost: every test's FLOPs),
@@ -155,61 +189,103 @@ __device__ __forceinline__ int near_pairs(const Frame &Tab, const LeafPair *__re
     return kNearFree;
 }
 
-// The steps marked in `word` (32 of the schedule's, from `base` on), in
-// order.  The lanes of a warp take the union of their steps together, so that
-// they read the same table entries and run the same code.  F: frame view, G:
-// gate centres.  Returns NearAnswer + 4 * FLOPs: on a collision those of the
-// whole check so far, else those beyond what the same steps cost with nothing hit
-// (negative where a gate was hit early and its leaves cost less).
-// T: the robot's tables.
-template <class T, class Frames>
-__device__ __noinline__ unsigned near_walk(const Frames F, const float4 *__restrict__ G, unsigned word, int base,
-                                           const EnvGrid *g, float pad, int extra)
+// A configuration, its marks and passed steps, by value.
+template <int D>
+struct NearCfg {
+    float q[D];
+};
+template <int W>
+struct NearMarks {
+    unsigned marked[W], passed[W];
+};
+
+// A frame in local memory, three 16-byte rows.
+struct NearFrame {
+    float4 r[3];
+    __device__ __forceinline__ void set(const Frame &f)
+    {
+        r[0] = make_float4(f.m[0], f.m[1], f.m[2], f.m[3]);
+        r[1] = make_float4(f.m[4], f.m[5], f.m[6], f.m[7]);
+        r[2] = make_float4(f.m[8], f.m[9], f.m[10], f.m[11]);
+    }
+};
+__device__ __forceinline__ Frame frame_at(const NearFrame *F, int i)   // i: joint's config index, -1 the world
 {
-    unsigned todo = __reduce_or_sync(__activemask(), word);
-    for (; todo; todo &= todo - 1) {
-        const int s = __ffs(todo) - 1;
-        if (!(word >> s & 1)) continue;
-        const NearStep e = T::steps()[base + s];
-        int h = kNearFree, c;
-        if (e.kind == 0) {
-            const GenEnvGroup gr = T::env_groups()[e.index];
-            bool go = true;
-            if (gr.gate >= 0) {
-                const float4 p = G[gr.gate];
-                const int a = near_env(g, p.x, p.y, p.z, p.w + pad, c);
-                if (a == kNearUnsure) return kNearUnsure;
-                extra += c;
-                go = a == kNearHit;
-            }
-            if (go)
-                for (int k = gr.first_block; k < gr.first_block + gr.nblocks && h == kNearFree; k++) {
-                    const GenLeafBlock b = T::leaf_blocks()[k];
-                    const Frame A = frame_at(F, b.frame + 1);
-                    for (int i = b.first; i < b.first + b.n && h == kNearFree; i++) {
-                        const float4 l = T::leaves()[i];
-                        float x, y, z;
-                        xform(A, l, x, y, z);
-                        h = near_env(g, x, y, z, l.w + pad, c);
+    if (i < 0) return world_frame();
+    const float4 a = F[i].r[0], b = F[i].r[1], c = F[i].r[2];
+    return Frame{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w}};
+}
+
+// The marked steps, in the schedule's order.  The lanes of a warp take the
+// union of their steps together, so that they read the same table entries
+// and run the same code.  extra: FLOPs of the passed steps' leaf pairs.
+// Returns NearAnswer + 4 * FLOPs: on a collision those of the whole check so
+// far, else those beyond what all steps cost with nothing hit (negative where
+// a gate was hit early and its leaves cost less).  T: the robot's tables.
+template <class T>
+__device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const NearMarks<T::kWords> m, int extra,
+                                              const EnvGrid *g, float pad)
+{
+    NearFrame F[T::kFrames];
+    float4 G[T::kGates];
+    T::frames(q.q, F, G);
+#pragma unroll 1
+    for (int w = 0; w < T::kWords; w++) {
+        const unsigned word = m.marked[w];
+        unsigned todo = __reduce_or_sync(__activemask(), word);
+#pragma unroll 1
+        for (; todo; todo &= todo - 1) {
+            const int s = __ffs(todo) - 1;
+            if (!(word >> s & 1)) continue;
+            const NearStep e = T::steps()[32 * w + s];
+            int h = kNearFree, c;
+            if (e.kind == 0) {
+                const GenEnvGroup gr = T::env_groups()[e.index];
+                bool go = true;
+                if (gr.gate >= 0) {
+                    const float4 p = G[gr.gate];
+                    const int a = near_env(g, p.x, p.y, p.z, p.w + pad, c);
+                    if (a == kNearUnsure) return kNearUnsure;
+                    extra += c;
+                    go = a == kNearHit;
+                }
+                if (go)
+                    for (int k = gr.first_block; k < gr.first_block + gr.nblocks && h == kNearFree; k++) {
+                        const GenLeafBlock b = T::leaf_blocks()[k];
+                        const Frame A = frame_at(F, b.frame);
+                        for (int i = b.first; i < b.first + b.n && h == kNearFree; i++) {
+                            const float4 l = T::leaves()[i];
+                            float x, y, z;
+                            xform(A, l, x, y, z);
+                            h = near_env(g, x, y, z, l.w + pad, c);
+                            extra += c;
+                        }
+                    }
+                extra -= g->cost * e.tests;
+            } else {
+                const GenSelfGroup gr = T::self_groups()[e.index];
+                const float4 a = G[gr.ga], b = G[gr.gb];
+                const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+                const int gate = near_verdict(dx * dx + dy * dy + dz * dz, (a.w + b.w) + 2.0f * pad);
+                if (gate == 2) return kNearUnsure;
+                if (gate == 1)
+                    for (int k = gr.first_block; k < gr.first_block + gr.nblocks && h == kNearFree; k++) {
+                        const NearPairBlock b = T::pair_blocks()[k];
+                        h = near_pairs(relative_frame(frame_at(F, b.fa), frame_at(F, b.fb)), T::pairs(), b, 2.0f * pad, c);
                         extra += c;
                     }
+            }
+            if (h == kNearUnsure) return kNearUnsure;
+            if (h == kNearHit) {   // the passed steps after this one were not reached
+                unsigned after = m.passed[w] & ~0u << s;
+                for (int v = w;;) {
+                    for (; after; after &= after - 1) extra -= kFlopPair * T::steps()[32 * v + __ffs(after) - 1].tests;
+                    if (++v >= T::kWords) break;
+                    after = m.passed[v];
                 }
-            extra -= g->cost * e.tests;
-        } else {
-            const GenSelfGroup gr = T::self_groups()[e.index];
-            const float4 a = G[gr.ga], b = G[gr.gb];
-            const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
-            const int gate = near_verdict(dx * dx + dy * dy + dz * dz, (a.w + b.w) + 2.0f * pad);
-            if (gate == 2) return kNearUnsure;
-            if (gate == 1)
-                for (int k = gr.first_block; k < gr.first_block + gr.nblocks && h == kNearFree; k++) {
-                    const NearPairBlock b = T::pair_blocks()[k];
-                    h = near_pairs(relative_frame(frame_at(F, b.fa + 1), frame_at(F, b.fb + 1)), T::pairs(), b, 2.0f * pad, c);
-                    extra += c;
-                }
+                return kNearHit + 4u * (unsigned)(g->cost * e.env + kFlopPair * e.self + extra);
+            }
         }
-        if (h == kNearUnsure) return kNearUnsure;
-        if (h == kNearHit) return kNearHit + 4u * (unsigned)(g->cost * e.env + kFlopPair * e.self + extra);
     }
     return kNearFree + 4u * (unsigned)extra;
 }

@@ -48,18 +48,19 @@ struct ValidateLaunch {
     static constexpr int kMaxThreads = 128, kMinBlocks = 8;
 };
 
-template <class Gen>
+template <class Gen, class Ctx>
 __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaunch<Gen>::kMinBlocks)
     k_validate_configs(const float4 *__restrict__ env, EnvCounts nc, const EnvGrid *grid,
                                                           const float *__restrict__ q, int64_t n,
-                                                          uint8_t *__restrict__ out, unsigned long long *work)
+                                                          uint8_t *__restrict__ out, unsigned long long *work, int spread)
 {
     extern __shared__ float4 s_env[];
     __shared__ unsigned long long s_bar;
     __shared__ EnvGrid s_grid;
     const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
-    CheckCtx ctx{{s_env, nc, gr}, 0.0f, nullptr};
+    Ctx ctx{};
+    ctx.env = EnvView{s_env, nc, gr};
     unsigned long long flops = 0, cfgs = 0;
     // The warp steps through the grid-stride loop together (a warp-uniform
     // trip count) and meets at __syncwarp after every configuration: lanes
@@ -67,10 +68,11 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
     // configuration out of step with the rest.  Blocks are whole warps (128
     // threads).  Baxter's table-form walk on 2^20 random configurations: 4.7
     // instead of 17.2 ms, 13.7 instead of 3.7 lanes active per instruction.
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w < n; w += stride) {
+    // spread: a warp takes 32 >> spread configurations at a time.
+    const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> spread;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> spread; w < n; w += stride) {
         const int64_t i = w + (threadIdx.x & 31u);
-        if (i < n) {
+        if (i < n && (threadIdx.x & 31u) < 32u >> spread) {
             float cfg[Gen::kDof];
             load_cfg<Gen::kDof>(q, i, cfg);
             ctx.work = 0;
@@ -83,50 +85,54 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
     add_work(work, flops, cfgs);
 }
 
-// One block per edge (grid-stride): thread t checks points k = t+1, t+1+blockDim, ...
-// MinBlocks > 0 builds it for that many resident 128-thread blocks per SM: 8
-// (at most 64 registers) is faster for 128-point edges (the Panda shelf
-// scene at g = 128: 1.79 vs 1.91 ms for 2^14 edges) and slower for the
-// 32-thread blocks of short edges, which keep the unconstrained build (0).
-template <class Gen, int MinBlocks>
-__global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
+// Edges, a warp per 32 points of one edge: points k = 32 c + lane + 1 of edge e
+// for item c * n + e.  out holds 1 for every edge when the kernel starts; a
+// warp that meets a collision writes 0, and a warp whose edge is already known
+// to collide skips its points.  Warps meet at no barrier (with a block per
+// edge, waiting for the block's slowest warp was a fifth of the time).
+// Chunk-major order: an edge's chunks run far apart, so that a later chunk
+// mostly finds the earlier ones' answer.
+template <class Gen>
+__global__ void __launch_bounds__(128, 6) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
                                                         const EnvGrid *grid,
                                                         const float *__restrict__ a, const float *__restrict__ b,
-                                                        int64_t n, int g, uint8_t *__restrict__ out,
-                                                        unsigned long long *work)
+                                                        int64_t n, int g, uint8_t *out, unsigned long long *work)
 {
     unsigned long long flops = 0, cfgs = 0;
     constexpr int D = Gen::kDof;
     extern __shared__ float4 s_env[];
-    __shared__ float s_a[D], s_step[D];
-    __shared__ int s_bad;
     __shared__ unsigned long long s_bar;
     __shared__ EnvGrid s_grid;
+    __shared__ int s_bad[4];
     const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
-    CheckCtx ctx{{s_env, nc, gr}, 0.0f, &s_bad};
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    volatile int *bad = &s_bad[warp];
+    CheckCtx ctx{{s_env, nc, gr}, 0.0f, bad};
     const float fg = (float)g;
-    for (int64_t e = blockIdx.x; e < n; e += gridDim.x) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_bad = 0;
-        if (threadIdx.x < D) {
-            const float av = __ldg(a + e * D + threadIdx.x);
-            s_a[threadIdx.x] = av;
-            s_step[threadIdx.x] = __fdiv_rn(__fsub_rn(__ldg(b + e * D + threadIdx.x), av), fg);
-        }
-        __syncthreads();
-        for (int k = threadIdx.x + 1; k <= g; k += blockDim.x) {
-            if (s_bad) break;
+    const int64_t items = n * ((g + 31) >> 5), stride = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t it = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; it < items; it += stride) {
+        const int64_t e = it % n;
+        const int k = 32 * (int)(it / n) + lane + 1;
+        if (lane == 0) *bad = *(volatile uint8_t *)(out + e) == 0;
+        __syncwarp();
+        if (k <= g && !*bad) {
             float cfg[D];
 #pragma unroll
-            for (int d = 0; d < D; d++) cfg[d] = __fadd_rn(s_a[d], __fmul_rn((float)k, s_step[d]));
+            for (int d = 0; d < D; d++) {
+                const float av = __ldg(a + e * D + d);
+                const float step = __fdiv_rn(__fsub_rn(__ldg(b + e * D + d), av), fg);
+                cfg[d] = __fadd_rn(av, __fmul_rn((float)k, step));
+            }
             ctx.work = 0;
-            if (!Gen::fkcc(cfg, ctx)) s_bad = 1;
+            if (!Gen::fkcc(cfg, ctx)) {
+                *bad = 1;
+                out[e] = 0;
+            }
             flops += ctx.work + Gen::kFkFlops;
             cfgs++;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) out[e] = s_bad ? 0 : 1;
+        __syncwarp();
     }
     add_work(work, flops, cfgs);
 }
@@ -142,7 +148,7 @@ __global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ e
     __shared__ EnvGrid s_grid;
     const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
-    CheckCtx ctx{{s_env, nc, gr}, 0.0f, nullptr};
+    SingleCheckCtx ctx{{{s_env, nc, gr}, 0.0f, nullptr}};
     // warp-uniform trip count, lanes meeting after every candidate (as in k_validate_configs)
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long tw = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); tw < g.tries; tw += stride) {
@@ -418,22 +424,30 @@ struct RobotKernels {
         if (n <= 0) return cudaSuccess;
         const int threads = 128;
         const size_t smem = (size_t)le.counts.records() * sizeof(float4);
-        k_validate_configs<Gen><<<grid_for(n, threads, le.sms, 16), threads, smem, st>>>(le.rec, le.counts, le.grid, q, n, out, le.work);
+        // A warp's time grows with the different groups its configurations
+        // come near (18 800 instructions for 32 random ones on the Panda shelf
+        // scene), so a call that cannot fill the GPU puts fewer in each: half
+        // as many while that leaves at most 8 warps per SM.
+        int spread = 0;
+        while (spread < 5 && (n << (spread + 1)) <= (int64_t)le.sms * 8 * 32) spread++;
+        const int blocks = grid_for(n << spread, threads, le.sms, 16);
+        if (spread >= 3)   // at most 4 configurations to a warp
+            k_validate_configs<Gen, SingleCheckCtx><<<blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, q, n, out,
+                                                                                   le.work, spread);
+        else
+            k_validate_configs<Gen, MixedCheckCtx><<<blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, q, n, out,
+                                                                                  le.work, spread);
         return cudaGetLastError();
     }
     static cudaError_t validate_edges(const LaunchEnv &le, const float *a, const float *b, int64_t n, int g,
                                       uint8_t *out, cudaStream_t st)
     {
         if (n <= 0) return cudaSuccess;
-        const int threads = g >= 128 ? 128 : ((g + 31) / 32) * 32;
         const size_t smem = (size_t)le.counts.records() * sizeof(float4);
-        int64_t blocks = n;
-        const int64_t cap = (int64_t)le.sms * (2048 / threads);
-        if (blocks > cap) blocks = cap;
-        if (threads == 128)
-            k_validate_edges<Gen, 8><<<(int)blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
-        else
-            k_validate_edges<Gen, 0><<<(int)blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
+        const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
+        if (e != cudaSuccess) return e;
+        k_validate_edges<Gen><<<grid_for(n * ((g + 31) / 32) * 32, 128, le.sms, 16), 128, smem, st>>>(
+            le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
         return cudaGetLastError();
     }
     static cudaError_t fk_spheres(const float *q, int64_t n, float *out, int sms, cudaStream_t st)

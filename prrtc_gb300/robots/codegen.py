@@ -481,19 +481,12 @@ def emit_cuda_checker(m: dict) -> str:
         for kind, gi in m["schedule"]:
             n = _env_tests(m, gi) if kind == "env" else 0
             ne, ns = ne + n, ns + (kind != "env")
-            w(f"    {{{0 if kind == 'env' else 1}, {gi}, {ne}, {ns}, {n}}},")
+            w(f"    {{{0 if kind == 'env' else 1}, {gi}, {ne}, {ns}, {n if kind == 'env' else len(m['self_groups'][gi]['pairs'])}}},")
         w("};")
         w(f"__device__ const NearPairBlock k{R}NearPair[{max(1, len(pblocks))}] = {{")
         for fa, fb, pf, n in pblocks or [(-1, -1, 0, 0)]:
             row, c, r = _rows(pair_rows[pf:pf + n])
             w(f"    {{{fa}, {fb}, {pf}, {n}, {{{', '.join(_lit(v) for v in [*c, r])}}}, {row}}},")
-        w("};")
-        w(f"struct {R}Near {{")
-        for name, type_, arr in (("steps", "NearStep", "NearStep"), ("env_groups", "GenEnvGroup", "EnvGroup"),
-                                 ("leaf_blocks", "GenLeafBlock", "LeafBlock"), ("leaves", "float4", "Leaf"),
-                                 ("self_groups", "GenSelfGroup", "SelfGroup"), ("pair_blocks", "NearPairBlock", "NearPair"),
-                                 ("pairs", "LeafPair", "Pair")):
-            w(f"    static __device__ __forceinline__ const {type_} *{name}() {{ return k{R}{arr}; }}")
         w("};")
     w("")
 
@@ -506,26 +499,45 @@ def emit_cuda_checker(m: dict) -> str:
         w("}")
         w("")
 
-    def fast_or(exact, near):
+    def fast_or(exact):
         """The fast form's answer, else the exact form's (on values the
         compiler cannot tell from new ones, so that it keeps none of the fast
         form's kinematics for them)."""
-        return [f"const int a = {near}(q, ctx);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
+        return ["const int a = near_check(q, ctx);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
                 "#pragma unroll", "for (int d = 0; d < kDof; d++) {", "    c[d] = q[d];",
-                '    asm volatile("" : "+f"(c[d]));', "}", f"return {exact}(c, ctx);"]
+                '    asm volatile("" : "+f"(c[d]));', "}", f"if constexpr (Ctx::kInlineExact) return {exact}(c, ctx);",
+                "Ctx own = ctx;   // the call must not force the caller's into memory",
+                f"const bool free = {exact}_call(c, own);", "ctx.work = own.work;", "return free;"]
 
     if table:
-        function("__device__ __forceinline__ bool fkcc_exact", tcode.lines)
-        if inline:
-            function("__device__ __forceinline__ bool fkcc_validate_exact", code.lines)
-        function("__device__ __forceinline__ int fkcc_near", _near_body(m, near_ids, store_late=False))
-        if inline:
-            function("__device__ __forceinline__ int fkcc_validate_near", _near_body(m, near_ids, store_late=True))
+        near_gates = near_ids
+        w(f"struct {R}Near {{")
+        w(f"    static constexpr int kDof = {m['dof']}, kFrames = {len(m['joints'])}, kGates = {len(near_gates)}, "
+          f"kWords = {(len(m['schedule']) + 31) // 32};")
+        for name_, type_, arr in (("steps", "NearStep", "NearStep"), ("env_groups", "GenEnvGroup", "EnvGroup"),
+                                  ("leaf_blocks", "GenLeafBlock", "LeafBlock"), ("leaves", "float4", "Leaf"),
+                                  ("self_groups", "GenSelfGroup", "SelfGroup"), ("pair_blocks", "NearPairBlock", "NearPair"),
+                                  ("pairs", "LeafPair", "Pair")):
+            w(f"    static __device__ __forceinline__ const {type_} *{name_}() {{ return k{R}{arr}; }}")
+        w("    static __device__ __forceinline__ void frames(const float *q, NearFrame *F, float4 *G)")
+        w("    {")
+        for line in _near_frames(m, near_gates):
+            w("        " + line)
+        w("    }")
+        w("};")
+        w("")
+        for exact, lines in [("fkcc_exact", tcode.lines)] + ([("fkcc_validate_exact", code.lines)] if inline else []):
+            function(f"__device__ __forceinline__ bool {exact}", lines)
+            function(f"__device__ __noinline__ bool {exact}_call", [f"return {exact}(q, ctx);"])
+        function("__device__ __forceinline__ int near_check_leaves", _near_body(m, near_gates, LEAF_MARKS))
+        function("__device__ __forceinline__ int near_check_gates", _near_body(m, near_gates, ALWAYS))
+        function("__device__ __forceinline__ int near_check",
+                 ["if constexpr (Ctx::kLeafMarks) return near_check_leaves(q, ctx);", "else return near_check_gates(q, ctx);"])
     w("// Returns true when configuration q is collision-free.")
-    function("__device__ __forceinline__ bool fkcc", fast_or("fkcc_exact", "fkcc_near") if table else code.lines)
+    function("__device__ __forceinline__ bool fkcc", fast_or("fkcc_exact") if table else code.lines)
     w("// The same verdicts for the stand-alone checker of single configurations.")
     function("__device__ __forceinline__ bool fkcc_validate",
-             fast_or("fkcc_validate_exact", "fkcc_validate_near") if table and inline else ["return fkcc(q, ctx);"])
+             fast_or("fkcc_validate_exact") if table and inline else ["return fkcc(q, ctx);"])
     w("// World centre and radius of every model sphere (model sphere order).")
     w("__device__ __forceinline__ void fk_spheres(const float *__restrict__ q, float4 *__restrict__ out)")
     w("{")
@@ -540,71 +552,92 @@ def emit_cuda_checker(m: dict) -> str:
 
 def _bounding_sphere(spheres):
     """(centre, radius) of a sphere around the given (centre, radius) spheres,
-    radius rounded up."""
+    the radius rounded up."""
     c = np.mean([s[0] for s in spheres], axis=0)
     for k in range(2000):          # towards the farthest one, by shrinking steps
-        d = [np.linalg.norm(np.asarray(x) - c) + r for x, r in spheres]
+        d = [round(float(np.linalg.norm(np.asarray(x) - c)) + r, 9) for x, r in spheres]
         i = int(np.argmax(d))
         v = np.asarray(spheres[i][0]) - c
         n = np.linalg.norm(v)
-        if n < 1e-12:
+        if n < 1e-9:
             break
         c = c + v / n * min(n, d[i] * 0.5 / (k + 2))
-    return [float(x) for x in c], float(max(np.linalg.norm(np.asarray(x) - c) + r for x, r in spheres)) + 1e-5
+    c = np.round(c, 4)
+    r = max(float(np.linalg.norm(np.asarray(x) - c)) + r for x, r in spheres)
+    return [float(x) for x in c], float(np.ceil(r * 1e5 + 1.0) / 1e5)
 
 
 GRID_UNIT = 512        # kGridUnit, device_common.cuh
+NEAR_PAD = 1e-4        # kNearPad, near_check.cuh
+LEAF_MARKS = 0.03      # gate pairs that overlap in this share of random configurations get leaf marks
+ALWAYS = 0.9           # and above this the gates are not asked first
 WIDE = 0.19            # spheres above EnvGrid::out_r (env_grid.cu: 0.95 x 0.2 m)
 CLUSTER = 3            # gate pairs of two frames that are worth a test of the frames' gates as a whole
 
 
-def _near_body(m, gate_ids, store_late):
-    """The fast form (near_check.cuh): frames, gate centres, the marks of the
-    schedule's steps that can hit, then the walk over those.  store_late: the
-    frames and centres that the walk reads are stored only by lanes that walk."""
+def _near_frames(m, gate_ids):
+    """Every frame and gate centre into the walk's arrays (near_resolve)."""
+    code = _Code()
+    fk = _FkGen(m, code)
+    sp, w = m["spheres"], code.lines.append
+    frames = {-1: "world_frame()"}
+    for jt in m["joints"]:
+        frames[jt["q"]] = _frame_arg(fk.frame(jt["q"]))
+        w(f"F[{jt['q']}].set({frames[jt['q']]});")
+    for sidx, gid in gate_ids.items():
+        w(f"G[{gid}] = gate_centre({frames[sp[sidx]['frame']]}, {_sphere_arg(sp[sidx])});")
+    return code.lines
+
+
+def _sphere_arg(s):
+    return f"make_float4({', '.join(_lit(float(np.float32(v))) for v in (*s['c'], s['r']))})"
+
+
+def _near_body(m, gate_ids, leaf_marks):
+    """The fast form (near_check.cuh): frames, gate centres and the marks of the
+    schedule's steps that can hit, in chain order; then the walk, for lanes
+    with marked steps.  Self groups whose gates overlap in at least this share
+    of random configurations get leaf marks."""
     R = m["robot"].capitalize()
     code = _Code()
     fk = _FkGen(m, code)
-    sp, nj, w = m["spheres"], len(m["joints"]), code.lines.append
+    sp, w = m["spheres"], code.lines.append
     w("const EnvGrid *grid = ctx.env.grid;")
     w("if (!grid || !(grid->lo[0] <= grid->hi[0])) return kNearUnsure;")
     w(f"if (!({' + '.join(f'fabsf(q[{d}])' for d in range(m['dof']))} < 100.0f)) return kNearUnsure;")
     for jt in m["joints"]:
         if jt["type"] != "revolute":
             w(f"if (fabsf(q[{jt['q']}]) > 4.0f) return kNearUnsure;")
-    frames = [fk.frame(jt["q"]) for jt in m["joints"]]
-    fexpr = {-1: "world_frame()"} | {jt["q"]: _frame_arg(T) for jt, T in zip(m["joints"], frames)}
-    w(f"FrameStore<Ctx, {nj + 1}> F(ctx);")
-    w(f"float4 G[{max(1, len(gate_ids))}];")
-    store = [f"F.set({jt['q'] + 1}, {_frame_arg(T)});" for jt, T in zip(m["joints"], frames)]
-    if not store_late:
-        code.lines += store
-        store = []
-    # gate centres in world coordinates, from the frames still in registers
-    for sidx, gid in gate_ids.items():
-        c = [float(np.float32(v)) for v in (*sp[sidx]["c"], sp[sidx]["r"])]
-        w(f"const float4 g{gid} = gate_centre({fexpr[sp[sidx]['frame']]}, make_float4({', '.join(_lit(v) for v in c)}));")
-        if store_late:
-            store.append(f"G[{gid}] = g{gid};")
-        else:
-            w(f"G[{gid}] = g{gid};")
-    w("const NearView near = near_view(ctx);")
     steps = m["schedule"]
     words = (len(steps) + 31) // 32
-    w("unsigned " + ", ".join(f"m{k} = 0" for k in range(words)) + ";")
+    w("const NearView near = near_view(ctx);")
+    w("unsigned " + ", ".join(f"m{k} = 0, p{k} = 0" for k in range(words)) + ";   // marked and passed steps")
+    w("int extra = 0;   // FLOPs of the passed steps' leaf pairs")
 
     def mark(s, cond):
         return f"m{s >> 5} |= {cond} ? {hex(1 << (s & 31))}u : 0u;"
 
-    pairs = {}
+    env_of = {}     # sphere -> environment steps that it gates
     for s, (kind, gi) in enumerate(steps):
         if kind == "env":
             g = m["env_groups"][gi]
             for sidx in ([g["gate"]] if g["gate"] >= 0 else g["leaves"]):
-                r = np.float32(sp[sidx]["r"])
-                units = int(np.ceil(float(r) * GRID_UNIT))
-                w(mark(s, f"may_hit_env{'_wide' if r >= WIDE else ''}(near, g{gate_ids[sidx]}, {units})"))
-        else:
+                env_of.setdefault(sidx, []).append(s)
+    fexpr = {-1: "world_frame()"}
+    for f in [-1] + [jt["q"] for jt in m["joints"]]:
+        if f >= 0:
+            fexpr[f] = _frame_arg(fk.frame(f))
+        for sidx, gid in gate_ids.items():
+            if sp[sidx]["frame"] != f:
+                continue
+            w(f"const float4 g{gid} = gate_centre({fexpr[f]}, {_sphere_arg(sp[sidx])});")
+            r = np.float32(sp[sidx]["r"])
+            for s in env_of.get(sidx, []):
+                w(mark(s, f"may_hit_env{'_wide' if r >= WIDE else ''}(near, g{gid}, {int(np.ceil(float(r) * GRID_UNIT))})"))
+
+    pairs = {}
+    for s, (kind, gi) in enumerate(steps):
+        if kind != "env":
             a, b = m["self_groups"][gi]["gate"]
             key = tuple(sp[x]["frame"] if sp[x]["frame"] >= 0 else ("world", x) for x in (a, b))
             pairs.setdefault(key, []).append((s, a, b))
@@ -621,34 +654,105 @@ def _near_body(m, gate_ids, store_late):
             w(f"const float4 {clusters[name]} = gate_centre({fexpr[key]}, make_float4({', '.join(_lit(v) for v in [*c, r])}));")
         return clusters[name]
 
+    often = _gate_rates(m)
+
+    def test(s, a, b):
+        """The mark of self step s (gates a, b): by its gates, or, where those
+        overlap often, by its leaves."""
+        gi = steps[s][1]
+        gates = f"may_hit_pair(near, g{gate_ids[a]}, g{gate_ids[b]})"
+        if often[gi] < leaf_marks:
+            return [mark(s, gates)]
+        lines = []
+        for frame, balls in _leaf_marks(m, gi):
+            for (f, c, r), limits in balls:
+                ball = f"gate_centre({fexpr[f]}, make_float4({', '.join(_lit(v) for v in [*c, r])}))"
+                lines.append(f"{{ const float4 p = local_point({fexpr[frame]}, {ball});")
+                lines += [f"  n |= near_leaf(p, {', '.join(_lit(v) for v in row)});" for row in limits]
+                lines.append("}")
+        bit, k = f"{hex(1 << (s & 31))}u", s >> 5
+        body = ["    bool n = near.wide || h == 2;", *("    " + x for x in lines), f"    if (n) m{k} |= {bit};",
+                f"    else if (h) p{k} |= {bit}, extra += kFlopPair * {len(m['self_groups'][gi]['pairs'])};", "}"]
+        head = f"const int h = near_gate(near, g{gate_ids[a]}, g{gate_ids[b]});"
+        if often[gi] > ALWAYS:
+            return [f"{{   {head}", *body]
+        return [f"if ({head[:-1]}) {{", *body]
+
     for (ka, kb), list_ in pairs.items():
-        test = [mark(s, f"may_hit_pair(near, g{gate_ids[a]}, g{gate_ids[b]})") for s, a, b in list_]
+        tests = [x for s, a, b in list_ for x in test(s, a, b)]
         if len(list_) >= CLUSTER:
             ca = cluster(ka, sorted({a for _, a, _ in list_}))
             cb = cluster(kb, sorted({b for _, _, b in list_}))
             w(f"if (may_hit_pair(near, {ca}, {cb})) {{")
-            code.lines += ["    " + t for t in test]
+            code.lines += ["    " + t for t in tests]
             w("}")
         else:
-            code.lines += test
+            code.lines += tests
     any_ = " | ".join(f"m{k}" for k in range(words))
     env_total = sum(_env_tests(m, gi) for kind, gi in steps if kind == "env")
     self_total = sum(kind != "env" for kind, _ in steps)
-    w("int extra = 0;")
     w(f"if ({any_}) {{")
     w("    if (ctx.stop()) return kNearFree;")
-    code.lines += ["    " + t for t in store]
-    for k in range(words):
-        w(f"    if (m{k}) {{")
-        w(f"        const unsigned a = near_walk<{R}Near>(F.view(), G, m{k}, {32 * k}, grid, ctx.pad, extra);")
-        w("        if ((a & 3u) == kNearHit) ctx.work += a >> 2;")
-        w("        if ((a & 3u) != kNearFree) return (int)(a & 3u);")
-        w("        extra = (int)a >> 2;")
-        w("    }")
+    w(f"    const unsigned a = near_resolve<{R}Near>(NearCfg<kDof>{{{{{', '.join(f'q[{d}]' for d in range(m['dof']))}}}}},")
+    w(f"        NearMarks<{words}>{{{{{', '.join(f'm{k}' for k in range(words))}}}, {{{', '.join(f'p{k}' for k in range(words))}}}}}, "
+      "extra, grid, ctx.pad);")
+    w("    if ((a & 3u) == kNearHit) ctx.work += a >> 2;")
+    w("    if ((a & 3u) != kNearFree) return (int)(a & 3u);")
+    w("    extra = (int)a >> 2;")
     w("}")
     w(f"ctx.work += (unsigned)(grid->cost * {env_total} + kFlopPair * {self_total} + extra);")
     w("return kNearFree;")
     return code.lines
+
+
+def _gate_rates(m):
+    """Share of random configurations in which each self group's gates overlap."""
+    from .. import scenes
+    q = scenes._uniform_configs(m["robot"], scenes.Rng(1), 2048)
+    C = scenes.sphere_centres(m["robot"], q)
+    r = [s["r"] for s in m["spheres"]]
+    return [float((((C[a] - C[b]) ** 2).sum(-1) < (r[a] + r[b]) ** 2).mean()) for a, b in (g["gate"] for g in m["self_groups"])]
+
+
+def _balls(spheres):
+    """A few balls [(centre, radius)] around (centre, radius) spheres, tighter
+    than one: grouped by the nearest of seeds that are far from one another."""
+    P = np.array([c for c, _ in spheres])
+    k = min(len(P), 3) if len(P) > 2 else 1
+    seeds = [int(np.argmax(((P - P.mean(0)) ** 2).sum(1)))]
+    while len(seeds) < k:
+        seeds.append(int(np.argmax(np.min([((P - P[i]) ** 2).sum(1) for i in seeds], axis=0))))
+    cen = P[seeds]
+    for _ in range(8):
+        of = np.argmin(((P[:, None] - cen) ** 2).sum(-1).round(9), 1)
+        cen = np.array([P[of == i].mean(0) if (of == i).any() else cen[i] for i in range(k)])
+    return [_bounding_sphere([spheres[j] for j in range(len(P)) if of[j] == i]) for i in range(k) if (of == i).any()]
+
+
+def _leaf_marks(m, gi):
+    """Leaf tests of a self group: [(frame, [((ball's frame, centre, radius),
+    [(-2 a, limit) per leaf a of `frame`])])], see near_check.cuh."""
+    sp = m["spheres"]
+    f32 = lambda v: float(np.float32(v))  # noqa: E731
+    sph = lambda i: ([f32(x) for x in sp[i]["c"]], f32(sp[i]["r"]))  # noqa: E731
+    A, B = (sorted({p[k] for p in m["self_groups"][gi]["pairs"]}) for k in (0, 1))
+    if len(A) > len(B):
+        A, B = B, A      # the longer list is enclosed in balls
+    balls = []
+    for f in sorted({sp[i]["frame"] for i in B}):
+        balls += [(f, c, r) for c, r in _balls([sph(i) for i in B if sp[i]["frame"] == f])]
+    out = []
+    for f in sorted({sp[i]["frame"] for i in A}):
+        tests = []
+        for ball in balls:
+            rows = []
+            for i in (i for i in A if sp[i]["frame"] == f):
+                a, r = sph(i)
+                s = r + ball[2] + 2 * NEAR_PAD + 2e-5
+                rows.append([-2 * x for x in a] + [round(s * s - sum(x * x for x in a) + 2e-6, 7)])
+            tests.append((ball, rows))
+        out.append((f, tests))
+    return out
 
 
 def _rows(rows):
@@ -663,9 +767,7 @@ def _rows(rows):
     if row < 3 or len(a) % row or len(a) // row > 32 or any(
             a[k] != a[k - k % row] or b[k] != b[k % row] for k in range(len(a))):
         return 0, [0.0, 0.0, 0.0], 0.0
-    c, r = _bounding_sphere([(np.array(f(x)), float(np.float32(y))) for x, y in b[:row]])
-    c = f(c)   # as the table holds it
-    return row, c, max(float(np.linalg.norm(np.array(f(x)) - np.array(c))) + float(np.float32(y)) for x, y in b[:row]) + 1e-5
+    return row, *_bounding_sphere([(np.array(f(x)), float(np.float32(y))) for x, y in b[:row]])
 
 
 def _env_tests(m, gi):
