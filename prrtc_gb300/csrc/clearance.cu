@@ -14,25 +14,6 @@
 
 namespace prrtc {
 
-// Every waypoint of every path: one thread per waypoint, blocks of 64
-// waypoints of one path, the path's obstacles staged in shared memory.
-__global__ void __launch_bounds__(64) k_path_cost_grad(ClrModel M, const ClrEnv *__restrict__ envs, int waypoints,
-                                                      const float *__restrict__ q, float margin,
-                                                      float *__restrict__ cost, float *__restrict__ grad)
-{
-    extern __shared__ float4 s_env[];
-    __shared__ unsigned long long s_bar;
-    const int path = blockIdx.y;
-    const ClrEnv pe = envs[path];
-    stage_env_bulk(s_env, pe.rec, pe.n.records(), &s_bar);
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= waypoints) return;
-    const size_t row = (size_t)path * waypoints + w;
-    float g[kClrMaxJoints];
-    cost[row] = clr::cost_grad(M, ClrEnv{s_env, pe.n}, q + row * M.dof, margin, 1.0f, g);
-    for (int d = 0; d < M.dof; d++) grad[row * M.dof + d] = g[d];
-}
-
 // One thread per query: the smallest clearance of its start and goals.
 __global__ void __launch_bounds__(64) k_query_clearance(ClrModel M, const BatchQueryDesc *__restrict__ queries,
                                                        const float *__restrict__ cfg, int n, float *__restrict__ score)
@@ -76,19 +57,25 @@ static prrtc_status model_on_device(Ctx *c, prrtc_robot robot, ClrModel *model)
     ClearanceState *cs = c->clearance;
     if (!cs->tables[robot]) {
         const ClrHostModel &h = clr_host_model(robot);
-        const void *src[7] = {h.joints.data(), h.parent.data(), h.leaf.data(),     h.leaf_joint.data(),
-                              h.pa.data(),     h.pb.data(),     h.pair_joint.data()};
-        const size_t bytes[7] = {h.joints.size() * sizeof(prrtc_joint_def), h.parent.size() * sizeof(int),
-                                 h.leaf.size() * sizeof(float4),            h.leaf_joint.size() * sizeof(int),
-                                 h.pa.size() * sizeof(float4),              h.pb.size() * sizeof(float4),
-                                 h.pair_joint.size() * sizeof(int2)};
-        size_t off[7], total = 0;
-        for (int k = 0; k < 7; k++) {
+        constexpr int kParts = 13;
+        const void *src[kParts] = {h.joints.data(),     h.parent.data(),     h.leaf.data(),       h.leaf_joint.data(),
+                                   h.pa.data(),         h.pb.data(),         h.pair_joint.data(), h.chain.data(),
+                                   h.leaf_sets.data(),  h.set_leaves.data(), h.pair_sets.data(),  h.pair_rows.data(),
+                                   h.pair_spheres.data()};
+        const size_t bytes[kParts] = {h.joints.size() * sizeof(prrtc_joint_def), h.parent.size() * sizeof(int),
+                                      h.leaf.size() * sizeof(float4),            h.leaf_joint.size() * sizeof(int),
+                                      h.pa.size() * sizeof(float4),              h.pb.size() * sizeof(float4),
+                                      h.pair_joint.size() * sizeof(int2),        h.chain.size() * sizeof(unsigned),
+                                      h.leaf_sets.size() * sizeof(ClrLeafSet),   h.set_leaves.size() * sizeof(float4),
+                                      h.pair_sets.size() * sizeof(ClrPairSet),   h.pair_rows.size() * sizeof(ClrPairRow),
+                                      h.pair_spheres.size() * sizeof(float4)};
+        size_t off[kParts], total = 0;
+        for (int k = 0; k < kParts; k++) {
             off[k] = total;
             total += al16(std::max<size_t>(bytes[k], 16));
         }
         std::vector<char> blob(total, 0);
-        for (int k = 0; k < 7; k++)
+        for (int k = 0; k < kParts; k++)
             if (bytes[k]) memcpy(blob.data() + off[k], src[k], bytes[k]);
         char *d = nullptr;
         if (cudaMalloc(&d, total) != cudaSuccess) {
@@ -112,6 +99,14 @@ static prrtc_status model_on_device(Ctx *c, prrtc_robot robot, ClrModel *model)
         m.pair_a = (const float4 *)(d + off[4]);
         m.pair_b = (const float4 *)(d + off[5]);
         m.pair_joint = (const int2 *)(d + off[6]);
+        m.n_leaf_sets = (int)h.leaf_sets.size();
+        m.n_pair_sets = (int)h.pair_sets.size();
+        m.chain = (const unsigned *)(d + off[7]);
+        m.leaf_sets = (const ClrLeafSet *)(d + off[8]);
+        m.set_leaves = (const float4 *)(d + off[9]);
+        m.pair_sets = (const ClrPairSet *)(d + off[10]);
+        m.pair_rows = (const ClrPairRow *)(d + off[11]);
+        m.pair_spheres = (const float4 *)(d + off[12]);
         cs->tables[robot] = d;
     }
     *model = cs->model[robot];
@@ -131,7 +126,7 @@ static prrtc_status prepare(Ctx *c, prrtc_robot robot, const prrtc_env *const *e
     for (int i = 0; i < n_paths; i++) {
         const Env *e = reinterpret_cast<const Env *>(envs[i]);
         if (!e) return c->fail(PRRTC_EINVAL, "clearance: environment of path %d is null", i);
-        table[i] = ClrEnv{e->dev, e->counts};
+        table[i] = ClrEnv{e->dev, e->counts, e->grid};
         mr = std::max(mr, e->counts.records());
     }
     // earlier work on the context's stream may still read the old table
@@ -196,10 +191,9 @@ extern "C" prrtc_status prrtc_path_cost_grad(prrtc_ctx *ctx, prrtc_robot robot, 
         (s = c->device_view(cost, rows * sizeof(float), 1, false, &dcost)) ||
         (s = c->device_view(grad, rows * M.dof * sizeof(float), 2, false, &dgrad)))
         return s;
-    const dim3 grid((waypoints + 63) / 64, n_paths);
-    k_path_cost_grad<<<grid, 64, (size_t)max_rec * sizeof(float4), c->stream>>>(
-        M, c->clearance->envs, waypoints, (const float *)dq, margin, (float *)dcost, (float *)dgrad);
-    if ((s = c->cuda(cudaGetLastError(), "path_cost_grad: launch"))) return s;
+    if ((s = c->cuda(ops->path_cost_grad(M, c->clearance->envs, (int64_t)rows, waypoints, (const float *)dq, margin,
+                                         (float *)dcost, (float *)dgrad, c->stream), "path_cost_grad: launch")))
+        return s;
     c->launches++;
     if (dcost != cost && (s = c->cuda(cudaMemcpyAsync(cost, dcost, rows * sizeof(float), cudaMemcpyDeviceToHost,
                                                       c->stream),
@@ -261,6 +255,7 @@ extern "C" prrtc_status prrtc_smooth_paths(prrtc_ctx *ctx, prrtc_robot robot, co
     P.envs = c->clearance->envs;
     P.n_paths = n_paths;
     P.waypoints = waypoints;
+    P.sms = c->sms;
     P.q = (float *)dq;
     P.s = ClrSmooth{st.margin, st.step, st.cost_weight, st.smooth_weight, st.steps, st.granularity, st.shortcut_rounds};
     P.accepted = (uint8_t *)dacc;

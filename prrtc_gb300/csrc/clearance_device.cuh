@@ -37,6 +37,23 @@ namespace prrtc {
 
 constexpr int kClrMaxJoints = 14;
 
+// Leaf spheres of one frame that lie in a ball (frame coordinates), set_leaves[first ..].
+struct ClrLeafSet {
+    float4 ball;
+    int joint, first, n, pad_;
+};
+// The self-collision pairs of two frames: the balls around either side, and rows
+// of pairs, one sphere a each.
+struct ClrPairSet {
+    float4 ball_a, ball_b;
+    int ja, jb, first, n;   // rows
+};
+struct ClrPairRow {
+    float4 a;
+    float4 ball;            // around the row's spheres b
+    int first, n, pad_[2];  // pair_spheres[first ..]
+};
+
 // A robot's collision model in the layout the clearance kernels read: every
 // index is a position in these tables (joints in chain order, parents first).
 struct ClrModel {
@@ -47,12 +64,21 @@ struct ClrModel {
     const int *leaf_joint;     // table position of each leaf's joint, -1 = world
     const float4 *pair_a, *pair_b;
     const int2 *pair_joint;
+    // the same leaves and pairs for the four-lane form (clearance_eval.cuh)
+    int n_leaf_sets, n_pair_sets;
+    const unsigned *chain;     // per joint: itself and its ancestors, a bit each
+    const ClrLeafSet *leaf_sets;
+    const float4 *set_leaves;
+    const ClrPairSet *pair_sets;
+    const ClrPairRow *pair_rows;
+    const float4 *pair_spheres;
 };
 
 // One path's obstacles (device records, layout of device_common.cuh).
 struct ClrEnv {
     const float4 *rec;
     EnvCounts n;
+    const EnvGrid *grid = nullptr;
 };
 
 // Smoothing settings as the kernels read them (prrtc_smooth_settings).
@@ -65,7 +91,7 @@ struct ClrSmooth {
 struct ClrLaunch {
     ClrModel M;
     const ClrEnv *envs;       // [n_paths]
-    int n_paths, waypoints;
+    int n_paths, waypoints, sms;
     float *q;                 // [n_paths][waypoints][dof], rewritten for accepted paths
     float lo[kClrMaxJoints], hi[kClrMaxJoints];   // joint limits
     ClrSmooth s;

@@ -3,19 +3,20 @@
 #pragma once
 
 #include "clearance_device.cuh"
+#include "clearance_eval.cuh"
 #include "planner_device.cuh"
 
 namespace prrtc {
 
 // Deterministic block sum (fixed blockDim, fixed order); every thread gets it.
-__device__ __forceinline__ float block_sum(float v, float *s_red)
+__device__ __forceinline__ double block_sum(double v, double *s_red)
 {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
     __syncthreads();
     if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
     __syncthreads();
-    float t = 0.0f;
+    double t = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s_red[w];
     return t;
 }
@@ -32,34 +33,55 @@ __device__ __forceinline__ float block_sum(float v, float *s_red)
 // `granularity` points per edge (a + k ((b - a) / g), k = 1..g, as the
 // planner interpolates); it is written back only if every point is free, so a
 // rejected path is left exactly as it came in.
+// Four lanes evaluate a waypoint (clearance_eval.cuh), all threads check points.
 template <class Gen>
-__global__ void __launch_bounds__(128) k_smooth_paths(const ClrLaunch P)
+__host__ __device__ constexpr size_t smooth_eval_offset(int records, int waypoints)
+{
+    return (records * sizeof(float4) + 2 * sizeof(float) * waypoints * Gen::kDof + 15) & ~(size_t)15;
+}
+
+template <class Gen>
+__global__ void __launch_bounds__(256) k_smooth_paths(const ClrLaunch P)
 {
     constexpr int D = Gen::kDof;
     extern __shared__ float4 s_dyn[];
     __shared__ int s_bad;
-    __shared__ float s_red[4];
+    __shared__ double s_red[8];
     __shared__ unsigned long long s_bar;
+    __shared__ EnvGrid s_grid;
+    constexpr int NJ = Gen::kFrames - 1, SLOTS = (Gen::kFrames + 2) / 4;
     const int path = blockIdx.x;
     const int W = P.waypoints;
     const ClrEnv pe = P.envs[path];
     const int R = pe.n.records();
     float *s_q = reinterpret_cast<float *>(s_dyn + R);
     float *s_g = s_q + W * D;
+    auto *s_eval = reinterpret_cast<clr::EvalScratch<NJ> *>(reinterpret_cast<char *>(s_dyn) + smooth_eval_offset<Gen>(R, W));
     float *gq = P.q + (size_t)path * W * D;
     for (int i = threadIdx.x; i < W * D; i += blockDim.x) s_q[i] = gq[i];
+    const EnvGrid *gr = stage_grid(&s_grid, pe.grid, s_dyn, threadIdx.x, blockDim.x);
     stage_env_bulk(s_dyn, pe.rec, R, &s_bar);   // synchronises the block
-    const ClrEnv e{s_dyn, pe.n};
+    const ClrEnv e{s_dyn, pe.n, gr};
     const ClrSmooth s = P.s;
-    CheckCtx ctx{EnvView{e.rec, e.n}, 0.0f, &s_bad};
-    if (P.cost_before) {   // the cost of the path as given
-        float cost = 0.0f;
-        for (int w = threadIdx.x; w < W; w += blockDim.x) {
-            float g[kClrMaxJoints];
-            cost += clr::cost_grad(P.M, e, s_q + w * D, s.margin, s.cost_weight, g);
+    CheckCtx ctx{EnvView{e.rec, e.n, gr}, 0.0f, &s_bad};
+    const int group = threadIdx.x >> 2, groups = blockDim.x >> 2, l = threadIdx.x & 3;
+    // every waypoint's cost (returned summed over this thread's) and gradient
+    auto evaluate = [&](auto &&store) {
+        double cost = 0.0;
+        for (int w0 = 0; w0 < W; w0 += groups) {
+            const int w = w0 + group;
+            double gr[SLOTS];
+            const double c = clr::eval<Gen>(s_eval[group], P.M, e, s_q + (w < W ? w : 0) * D, w < W, s.margin, gr);
+            if (w < W) {
+                if (l == 0) cost += c;
+                store(w, gr);
+            }
         }
-        const float total = block_sum(cost, s_red);
-        if (threadIdx.x == 0) P.cost_before[path] = total;
+        return cost;
+    };
+    if (P.cost_before) {   // the cost of the path as given
+        const double total = block_sum(evaluate([](int, const double(&)[SLOTS]) {}), s_red);
+        if (threadIdx.x == 0) P.cost_before[path] = (float)total;
     }
     const int gs = max(1, s.granularity / 4);
     for (int r = 0; r < s.shortcut_rounds && W > 2; r++) {
@@ -92,19 +114,19 @@ __global__ void __launch_bounds__(128) k_smooth_paths(const ClrLaunch P)
         __syncthreads();
     }
     for (int it = 0; it <= s.steps; it++) {
-        float cost = 0.0f;
-        for (int w = threadIdx.x; w < W; w += blockDim.x) {
-            float g[kClrMaxJoints];
-            cost += clr::cost_grad(P.M, e, s_q + w * D, s.margin, s.cost_weight, g);
-            if (w > 0 && w < W - 1)
+        const double cost = evaluate([&](int w, const double(&gr)[SLOTS]) {
+            if (w == 0 || w == W - 1) return;
 #pragma unroll
-                for (int d = 0; d < D; d++)
-                    s_g[w * D + d] =
-                        g[d] + s.smooth_weight * (2.0f * s_q[w * D + d] - s_q[(w - 1) * D + d] - s_q[(w + 1) * D + d]);
-        }
+            for (int t = 0; t < SLOTS; t++)
+                if (l + 4 * t < NJ) {
+                    const int d = P.M.joints[l + 4 * t].q;
+                    s_g[w * D + d] = (float)((double)s.cost_weight * gr[t]) +
+                                     s.smooth_weight * (2.0f * s_q[w * D + d] - s_q[(w - 1) * D + d] - s_q[(w + 1) * D + d]);
+                }
+        });
         if (it == s.steps) {
-            const float total = block_sum(cost, s_red);
-            if (threadIdx.x == 0 && P.cost_after) P.cost_after[path] = total;
+            const double total = block_sum(cost, s_red);
+            if (threadIdx.x == 0 && P.cost_after) P.cost_after[path] = (float)total;
         }
         __syncthreads();
         if (it == s.steps) break;

@@ -212,6 +212,8 @@ size_t env_grid_bytes(int cells);
 cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st);
 
 struct ClrLaunch;   // clearance_device.cuh
+struct ClrModel;
+struct ClrEnv;
 struct Ctx;         // context.h
 
 // score[i] = smallest clearance (metres, float32 screen) of query i's start or
@@ -229,6 +231,8 @@ struct RobotOps {
     cudaError_t (*solve_plain)(const PlainParams &, int threads, cudaStream_t);
     cudaError_t (*solve_batch)(const BatchParams &, int blocks, int warps_per_block, cudaStream_t);
     int (*batch_occupancy)(int warps_per_block, int env_records, int shared_frames);   // resident blocks per SM
+    cudaError_t (*path_cost_grad)(const ClrModel &, const ClrEnv *envs, int64_t rows, int waypoints, const float *q,
+                                  float margin, float *cost, float *grad, cudaStream_t);
     cudaError_t (*smooth_paths)(const ClrLaunch &, size_t env_bytes, cudaStream_t);
     cudaError_t (*goal_flags)(const LaunchEnv &, const GoalQuery &, uint8_t *flags, cudaStream_t);
 };

@@ -493,13 +493,23 @@ struct RobotKernels {
         k_goal_flags<Gen><<<grid_for(g.tries, 128, le.sms, 16), 128, smem, st>>>(le.rec, le.counts, le.grid, g, flags);
         return cudaGetLastError();
     }
+    static cudaError_t path_cost_grad(const ClrModel &M, const ClrEnv *envs, int64_t rows, int waypoints, const float *q,
+                                      float margin, float *cost, float *grad, cudaStream_t st)
+    {
+        if (rows <= 0) return cudaSuccess;
+        k_path_cost_grad<Gen><<<(unsigned)((rows + 15) / 16), 64, 0, st>>>(M, envs, rows, waypoints, q, margin, cost, grad);
+        return cudaGetLastError();
+    }
     static cudaError_t smooth_paths(const ClrLaunch &P, size_t env_bytes, cudaStream_t st)
     {
         if (P.n_paths <= 0) return cudaSuccess;
-        const size_t smem = env_bytes + 2 * sizeof(float) * (size_t)P.waypoints * Gen::kDof;
+        // few paths: 256 threads each (every waypoint of 64 at once); many:
+        // 128, for more of them on an SM
+        const int threads = P.n_paths <= 2 * P.sms && P.waypoints > 32 ? 256 : 128;
+        const size_t smem = smooth_eval_offset<Gen>((int)(env_bytes / sizeof(float4)), P.waypoints) +
+                            sizeof(clr::EvalScratch<Gen::kFrames - 1>) * (threads / 4);
         cudaError_t e = cudaFuncSetAttribute(k_smooth_paths<Gen>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        const int threads = P.waypoints <= 64 ? 64 : 128;
         k_smooth_paths<Gen><<<P.n_paths, threads, smem, st>>>(P);
         return cudaGetLastError();
     }
@@ -514,6 +524,7 @@ struct RobotKernels {
         o.solve_plain = &solve_plain;
         o.solve_batch = &solve_batch;
         o.batch_occupancy = &batch_occupancy;
+        o.path_cost_grad = &path_cost_grad;
         o.smooth_paths = &smooth_paths;
         o.goal_flags = &goal_flags;
         (void)dof_check;
@@ -544,6 +555,11 @@ struct RobotKernels {
         static __device__ __forceinline__ void fk_spheres(const float *q, float4 *out)              \
         {                                                                                           \
             NS::fk_spheres(q, out);                                                                 \
+        }                                                                                           \
+        template <class Dd>                                                                         \
+        static __device__ __forceinline__ void clr_rows(int i, const Dd *trig, float *hi, float *lo) \
+        {                                                                                           \
+            NS::clr_rows(i, trig, hi, lo);                                                          \
         }                                                                                           \
     };                                                                                              \
     }

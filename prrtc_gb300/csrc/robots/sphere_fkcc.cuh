@@ -53,6 +53,41 @@ __device__ __forceinline__ bool fkcc_validate(const float *__restrict__ q, Ctx &
     return fkcc(q, ctx);
 }
 
+// Row i (0..2) of every joint's world frame in pairs of floats, joint at table
+// position j at hi / lo[12 j + 4 i + k]; trig: cosine and sine of each joint's
+// angle, or its value (clearance_eval.cuh).
+template <class Dd>
+__device__ __forceinline__ void clr_rows(int i, const Dd *__restrict__ trig, float *__restrict__ hi, float *__restrict__ lo)
+{
+    const Dd a0_0{i == 0 ? 0.0f : i == 1 ? 1.0f : 0.0f, 0.0f};
+    const Dd a0_1{i == 0 ? 0.0f : i == 1 ? 0.0f : 1.0f, 0.0f};
+    const Dd a0_2{i == 0 ? 1.0f : i == 1 ? 0.0f : 0.0f, 0.0f};
+    const Dd a0_3{0.0f, 0.0f};
+    const Dd t0_3 = a0_3 + a0_2 * trig[0].h;
+    hi[0 + 4 * i] = a0_0.h, lo[0 + 4 * i] = a0_0.l;
+    hi[1 + 4 * i] = a0_1.h, lo[1 + 4 * i] = a0_1.l;
+    hi[2 + 4 * i] = a0_2.h, lo[2 + 4 * i] = a0_2.l;
+    hi[3 + 4 * i] = t0_3.h, lo[3 + 4 * i] = t0_3.l;
+    const Dd a1_0 = a0_1;
+    const Dd a1_1 = a0_2;
+    const Dd a1_2 = a0_0;
+    const Dd a1_3 = t0_3;
+    const Dd t1_3 = a1_3 + a1_2 * trig[2].h;
+    hi[12 + 4 * i] = a1_0.h, lo[12 + 4 * i] = a1_0.l;
+    hi[13 + 4 * i] = a1_1.h, lo[13 + 4 * i] = a1_1.l;
+    hi[14 + 4 * i] = a1_2.h, lo[14 + 4 * i] = a1_2.l;
+    hi[15 + 4 * i] = t1_3.h, lo[15 + 4 * i] = t1_3.l;
+    const Dd a2_0 = a1_1;
+    const Dd a2_1 = a1_2;
+    const Dd a2_2 = a1_0;
+    const Dd a2_3 = t1_3;
+    const Dd t2_3 = a2_3 + a2_2 * trig[4].h;
+    hi[24 + 4 * i] = a2_0.h, lo[24 + 4 * i] = a2_0.l;
+    hi[25 + 4 * i] = a2_1.h, lo[25 + 4 * i] = a2_1.l;
+    hi[26 + 4 * i] = a2_2.h, lo[26 + 4 * i] = a2_2.l;
+    hi[27 + 4 * i] = t2_3.h, lo[27 + 4 * i] = t2_3.l;
+}
+
 // World centre and radius of every model sphere (model sphere order).
 __device__ __forceinline__ void fk_spheres(const float *__restrict__ q, float4 *__restrict__ out)
 {

@@ -538,6 +538,16 @@ def emit_cuda_checker(m: dict) -> str:
     w("// The same verdicts for the stand-alone checker of single configurations.")
     function("__device__ __forceinline__ bool fkcc_validate",
              fast_or("fkcc_validate_exact") if table and inline else ["return fkcc(q, ctx);"])
+    w("// Row i (0..2) of every joint's world frame in pairs of floats, joint at table")
+    w("// position j at hi / lo[12 j + 4 i + k]; trig: cosine and sine of each joint's")
+    w("// angle, or its value (clearance_eval.cuh).")
+    w("template <class Dd>")
+    w("__device__ __forceinline__ void clr_rows(int i, const Dd *__restrict__ trig, float *__restrict__ hi, float *__restrict__ lo)")
+    w("{")
+    for line in _clr_rows(m):
+        w("    " + line)
+    w("}")
+    w("")
     w("// World centre and radius of every model sphere (model sphere order).")
     w("__device__ __forceinline__ void fk_spheres(const float *__restrict__ q, float4 *__restrict__ out)")
     w("{")
@@ -768,6 +778,38 @@ def _rows(rows):
             a[k] != a[k - k % row] or b[k] != b[k % row] for k in range(len(a))):
         return 0, [0.0, 0.0, 0.0], 0.0
     return row, *_bounding_sphere([(np.array(f(x)), float(np.float32(y))) for x, y in b[:row]])
+
+
+def _clr_rows(m):
+    """One row of every frame, fixed transforms folded (T = parent F Rz(q))."""
+    f32 = lambda v: float(np.float32(v))  # noqa: E731
+    out, w, rows = [], None, {}
+    w = out.append
+    for pos, jt in enumerate(m["joints"]):
+        F = [[f32(v) for v in r] for r in jt["F"]]
+        A = []
+        for k in range(4):
+            if jt["parent"] < 0:       # the world's row i is a unit vector
+                c = [F[r][k] for r in range(3)]
+                e = _lit(c[0]) if c[0] == c[1] == c[2] else f"i == 0 ? {_lit(c[0])} : i == 1 ? {_lit(c[1])} : {_lit(c[2])}"
+                w(f"const Dd a{pos}_{k}{{{e}, 0.0f}};")
+            else:
+                P = rows[jt["parent"]]
+                terms = [P[r] if F[r][k] == 1.0 else f"(-{P[r]})" if F[r][k] == -1.0 else f"{P[r]} * {_lit(F[r][k])}"
+                         for r in range(3) if F[r][k] != 0.0] + ([P[3]] if k == 3 else [])
+                w(f"const Dd a{pos}_{k} = {' + '.join(terms) if terms else 'Dd{0.0f, 0.0f}'};")
+            A.append(f"a{pos}_{k}")
+        if jt["type"] == "revolute":
+            w(f"const Dd c{pos} = trig[{2 * pos}], s{pos} = trig[{2 * pos + 1}];")
+            w(f"const Dd t{pos}_0 = c{pos} * {A[0]} + s{pos} * {A[1]}, t{pos}_1 = c{pos} * {A[1]} - s{pos} * {A[0]};")
+            T = [f"t{pos}_0", f"t{pos}_1", A[2], A[3]]
+        else:
+            w(f"const Dd t{pos}_3 = {A[3]} + {A[2]} * trig[{2 * pos}].h;")
+            T = [A[0], A[1], A[2], f"t{pos}_3"]
+        rows[jt["q"]] = T
+        for k in range(4):
+            w(f"hi[{12 * pos + k} + 4 * i] = {T[k]}.h, lo[{12 * pos + k} + 4 * i] = {T[k]}.l;")
+    return out
 
 
 def _env_tests(m, gi):
