@@ -212,9 +212,9 @@ template <class Ctx>
 __device__ __forceinline__ Ctx make_ctx(const EnvView &view, float pad, volatile int *stop, float4 *frames)
 {
     if constexpr (Ctx::kSharedFrames)
-        return Ctx{CheckCtx{view, pad, stop}, frames};
+        return Ctx{PlanCheckCtx{{view, pad, stop}}, frames};
     else
-        return Ctx{view, pad, stop};
+        return Ctx{{view, pad, stop}};
 }
 
 // Whole warp: check the g points of the edge in W (from + k * step),
@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(128, 3) k_rrtc_batch(const BatchParams P)
         auto validate = [&]() {
             return P.shared_frames
                        ? warp_validate<Gen, SharedCheckCtx>(W, W_frames + lane, P.granularity, P.edge_order, P.pad, C->work)
-                       : warp_validate<Gen, CheckCtx>(W, nullptr, P.granularity, P.edge_order, P.pad, C->work);
+                       : warp_validate<Gen, PlanCheckCtx>(W, nullptr, P.granularity, P.edge_order, P.pad, C->work);
         };
         float *nodes_s = P.nodes + (size_t)slot * 2 * D * P.cap;
         int *par_s = P.parents + (size_t)slot * 2 * P.cap;

@@ -44,6 +44,26 @@ struct alignas(16) NearPairBlock {
     int row;
 };
 
+// Sine and cosine to 1e-7 for |x| <= 100: x minus a multiple of pi / 2 (in three
+// parts, the first two products exact), then the Taylor series up to r^9 / r^10.
+// The exact form has the library's; the two forms' centres differ by less
+// than 1.5e-6 m (half of near_verdict's band).
+__device__ __forceinline__ void near_sincos(float x, float *s, float *c)
+{
+    const float k = rintf(x * 0.636619772f);
+    const float r = fmaf(-k, 0x1.0b4612p-34f, fmaf(-k, 0x1.b544p-16f, fmaf(-k, 0x1.921ep+0f, x)));
+    const float y = r * r;
+    float u = fmaf(y, 1.0f / 362880.0f, -1.0f / 5040.0f), v = fmaf(y, -1.0f / 3628800.0f, 1.0f / 40320.0f);
+    u = fmaf(y, u, 1.0f / 120.0f), v = fmaf(y, v, -1.0f / 720.0f);
+    u = fmaf(y, u, -1.0f / 6.0f), v = fmaf(y, v, 1.0f / 24.0f);
+    v = fmaf(y, v, -0.5f);
+    u = fmaf(r * y, u, r), v = fmaf(y, v, 1.0f);
+    const int n = (int)k;
+    const float a = n & 1 ? v : u, b = n & 1 ? u : v;
+    *s = n & 2 ? -a : a;
+    *c = (n + 1) & 2 ? -b : b;
+}
+
 // The environment as the marking code reads it.
 struct NearView {
     const EnvGrid *g;

@@ -596,7 +596,7 @@ def _near_frames(m, gate_ids):
         w(f"F[{jt['q']}].set({frames[jt['q']]});")
     for sidx, gid in gate_ids.items():
         w(f"G[{gid}] = gate_centre({frames[sp[sidx]['frame']]}, {_sphere_arg(sp[sidx])});")
-    return code.lines
+    return [line.replace("sincosf(", "near_sincos(") for line in code.lines]
 
 
 def _sphere_arg(s):
@@ -712,7 +712,7 @@ def _near_body(m, gate_ids, leaf_marks):
     w("}")
     w(f"ctx.work += (unsigned)(grid->cost * {env_total} + kFlopPair * {self_total} + extra);")
     w("return kNearFree;")
-    return code.lines
+    return [line.replace("sincosf(", "near_sincos(") for line in code.lines]
 
 
 def _gate_rates(m):
