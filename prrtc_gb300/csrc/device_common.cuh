@@ -262,6 +262,11 @@ __device__ __forceinline__ int env_cost(const EnvCounts &n, int k)
     return a * kFlopSphere + b * kFlopCapsule + c * kFlopZCapsule + d * kFlopCuboid + (k - d) * kFlopZCuboid;
 }
 
+__device__ __forceinline__ int env_cost_all(const EnvCounts &n)
+{
+    return n.ns * kFlopSphere + n.nc * kFlopCapsule + n.nzc * kFlopZCapsule + n.ncb * kFlopCuboid + n.nzb * kFlopZCuboid;
+}
+
 // Sphere against obstacle k: 0 no hit, 1 hit, 2 too near contact to tell
 // here.  The distance is the reference test's; what is left to the exact test
 // is a band around contact wider than any rounding: 3e-6 m (two forms of the
@@ -439,8 +444,10 @@ static __device__ __noinline__ int self_pairs(const Frame Tab, const LeafPair *_
 // counts).  Frames are indexed by joint config index + 1; F[0] is the world.
 
 struct GenSched {
-    int kind;    // 0 environment group, 1 self group
+    int kind;          // 0 environment group, 1 self group
     int index;
+    short env, self;   // sphere-environment and gate-pair tests of the steps up to and with this one, none hit
+    int tests;         // environment: sphere tests of this step when nothing hits; self: its leaf pairs
 };
 struct GenEnvGroup {
     int gate;             // gating sphere: index into the gate centres, -1 none
@@ -563,6 +570,8 @@ struct CheckCtx {
         rs += 2.0f * pad;
         return dx * dx + dy * dy + dz * dz - rs * rs < 0.0f;
     }
+    // FLOPs of a sphere tested against every obstacle
+    __device__ __forceinline__ int cost() const { return env.grid ? env.grid->cost : env_cost_all(env.n); }
     __device__ __forceinline__ bool stop() const { return stop_flag != nullptr && *stop_flag != 0; }
 };
 
@@ -605,8 +614,6 @@ struct FrameStore<Ctx, N, true> : SharedFrames {
     __device__ __forceinline__ explicit FrameStore(const Ctx &c) : SharedFrames{c.frames} {}
 };
 
-// The schedule of a table-form checker (see GenSched); returns true when free.
-// F is a frame view: a local array (const Frame *) or SharedFrames.
 // A gate sphere (x, y, z, r in frame T) in world coordinates, radius kept.
 __device__ __forceinline__ float4 gate_centre(const Frame &T, float4 c)
 {
@@ -615,42 +622,67 @@ __device__ __forceinline__ float4 gate_centre(const Frame &T, float4 c)
     return make_float4(x, y, z, c.w);
 }
 
+// Which steps of the schedule the exact form has to make, a bit each: marked
+// ones; passed ones are self groups whose gates overlap and whose leaves are
+// known not to (near_check.cuh); the others' gates are known not to hit.
+template <int W>
+struct StepMarks {
+    unsigned marked[W], passed[W];
+};
+
 // G: the world centres of the gate spheres, computed with the frames (the
-// same xform as a leaf's, so verdicts do not change).
-template <class Frames, class Ctx>
+// same xform as a leaf's, so verdicts do not change).  The steps that are not
+// made count as the reference makes them.  (Making all 388 of them cost a Baxter
+// lane that came too near contact 170 us, the time of a call of 16 to 1000 edges.)
+template <class Frames, class Ctx, int W>
 __device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restrict__ G, const GenSched *__restrict__ sched,
                                           int nsched,
                                           const GenEnvGroup *__restrict__ eg, const GenLeafBlock *__restrict__ lb,
                                           const float4 *__restrict__ leaves, const GenSelfGroup *__restrict__ sg,
                                           const GenPairBlock *__restrict__ pb, const LeafPair *__restrict__ pairs,
-                                          Ctx &ctx)
+                                          Ctx &ctx, const StepMarks<W> &marks)
 {
-    for (int s = 0; s < nsched; s++) {
-        const GenSched e = sched[s];
-        if (e.kind == 0) {
-            const GenEnvGroup g = eg[e.index];
-            bool go = true;
-            if (g.gate >= 0) {
-                const float4 c = G[g.gate];
-                go = ctx.env_hit(c.x, c.y, c.z, c.w);
+    const int cost = ctx.cost();
+    int known = 0;   // FLOPs of the steps made, as if nothing hit
+    for (int w = 0; w < W; w++)
+        for (unsigned todo = marks.marked[w] | marks.passed[w]; todo; todo &= todo - 1) {
+            const int s = 32 * w + __ffs(todo) - 1;
+            if (s >= nsched) break;
+            const GenSched e = sched[s];
+            bool hit = false;
+            if (e.kind == 0) {
+                known += cost * e.tests;
+                const GenEnvGroup g = eg[e.index];
+                bool go = true;
+                if (g.gate >= 0) {
+                    const float4 c = G[g.gate];
+                    go = ctx.env_hit(c.x, c.y, c.z, c.w);
+                }
+                if (go)
+                    for (int k = g.first_block; k < g.first_block + g.nblocks && !hit; k++) {
+                        const GenLeafBlock b = lb[k];
+                        hit = ctx.env_leaves(frame_at(F, b.frame + 1), leaves + b.first, b.n);
+                    }
+            } else if (marks.passed[w] >> (s & 31) & 1) {
+                ctx.work += kFlopPair * e.tests;
+            } else {
+                known += kFlopPair;
+                const GenSelfGroup g = sg[e.index];
+                const float4 a = G[g.ga], b = G[g.gb];
+                if (ctx.pair_hit(a.x - b.x, a.y - b.y, a.z - b.z, a.w + b.w))
+                    for (int k = g.first_block; k < g.first_block + g.nblocks && !hit; k++) {
+                        const GenPairBlock b = pb[k];
+                        hit = ctx.self_pairs(relative_frame(frame_at(F, b.fa + 1), frame_at(F, b.fb + 1)), pairs + b.first, b.n);
+                    }
             }
-            if (go)
-                for (int k = g.first_block; k < g.first_block + g.nblocks; k++) {
-                    const GenLeafBlock b = lb[k];
-                    if (ctx.env_leaves(frame_at(F, b.frame + 1), leaves + b.first, b.n)) return false;
-                }
-        } else {
-            const GenSelfGroup g = sg[e.index];
-            const float4 a = G[g.ga], b = G[g.gb];
-            if (ctx.pair_hit(a.x - b.x, a.y - b.y, a.z - b.z, a.w + b.w))
-                for (int k = g.first_block; k < g.first_block + g.nblocks; k++) {
-                    const GenPairBlock b = pb[k];
-                    if (ctx.self_pairs(relative_frame(frame_at(F, b.fa + 1), frame_at(F, b.fb + 1)), pairs + b.first, b.n))
-                        return false;
-                }
+            if (hit) {
+                ctx.work += (unsigned)(cost * e.env + kFlopPair * e.self - known);
+                return false;
+            }
+            if (ctx.stop()) return true;
         }
-        if (ctx.stop()) return true;
-    }
+    const GenSched last = sched[nsched - 1];
+    ctx.work += (unsigned)(cost * last.env + kFlopPair * last.self - known);
     return true;
 }
 

@@ -28,13 +28,6 @@ namespace prrtc {
 
 enum NearAnswer { kNearHit = 0, kNearFree = 1, kNearUnsure = 2 };
 
-// One step of the schedule for the fast form.
-struct NearStep {
-    int kind;          // 0 environment group, 1 self group
-    int index;
-    short env, self;   // sphere-environment and gate-pair tests of the steps up to and with this one, none hit
-    int tests;         // environment: sphere tests of this step when nothing hits; self: its leaf pairs
-};
 // Leaf pairs of one block (GenPairBlock).  row > 0: rows of `row` pairs with one
 // sphere a each, every row against the same spheres b, all of which lie in
 // the sphere `bound` of frame B.
@@ -209,16 +202,11 @@ __device__ __forceinline__ int near_pairs(const Frame &Tab, const LeafPair *__re
     return kNearFree;
 }
 
-// A configuration, its marks and passed steps, by value.
+// A configuration by value.
 template <int D>
 struct NearCfg {
     float q[D];
 };
-template <int W>
-struct NearMarks {
-    unsigned marked[W], passed[W];
-};
-
 // A frame in local memory, three 16-byte rows.
 struct NearFrame {
     float4 r[3];
@@ -243,7 +231,7 @@ __device__ __forceinline__ Frame frame_at(const NearFrame *F, int i)   // i: joi
 // far, else those beyond what all steps cost with nothing hit (negative where
 // a gate was hit early and its leaves cost less).  T: the robot's tables.
 template <class T>
-__device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const NearMarks<T::kWords> m, int extra,
+__device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const StepMarks<T::kWords> m, int extra,
                                               const EnvGrid *g, float pad)
 {
     NearFrame F[T::kFrames];
@@ -257,7 +245,7 @@ __device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const Ne
         for (; todo; todo &= todo - 1) {
             const int s = __ffs(todo) - 1;
             if (!(word >> s & 1)) continue;
-            const NearStep e = T::steps()[32 * w + s];
+            const GenSched e = T::steps()[32 * w + s];
             int h = kNearFree, c;
             if (e.kind == 0) {
                 const GenEnvGroup gr = T::env_groups()[e.index];

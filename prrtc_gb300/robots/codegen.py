@@ -356,7 +356,7 @@ def emit_cuda_checker(m: dict) -> str:
         for sidx, gid in gate_ids.items():
             code.lines.append(f"G[{gid}] = gate_centre({fexpr[sp[sidx]['frame']]}, k{R}Gate[{gid}]);")
         code.lines.append(f"return run_schedule(F.view(), G, k{R}Sched, {len(m['schedule'])}, k{R}EnvGroup, k{R}LeafBlock, k{R}Leaf, "
-                          f"k{R}SelfGroup, k{R}PairBlock, k{R}Pair, ctx);")
+                          f"k{R}SelfGroup, k{R}PairBlock, k{R}Pair, ctx, marks);")
         tcode = code
         code = _Code()              # the straight-line form, if any, goes to its own code
         fk = _FkGen(m, code)
@@ -437,8 +437,11 @@ def emit_cuda_checker(m: dict) -> str:
     if table:
         w("// the schedule in table form (run_schedule)")
         w(f"__device__ const GenSched k{R}Sched[{len(m['schedule'])}] = {{")
+        ne = ns = 0
         for kind, gi in m["schedule"]:
-            w(f"    {{{0 if kind == 'env' else 1}, {gi}}},")
+            n = _env_tests(m, gi) if kind == "env" else len(m["self_groups"][gi]["pairs"])
+            ne, ns = (ne + n, ns) if kind == "env" else (ne, ns + 1)
+            w(f"    {{{0 if kind == 'env' else 1}, {gi}, {ne}, {ns}, {n}}},")
         w("};")
         lblocks, eg_rows = [], []
         for gi, g in enumerate(m["env_groups"]):
@@ -476,13 +479,6 @@ def emit_cuda_checker(m: dict) -> str:
             w(f"    {{{fa}, {fb}, {pf}, {n}}},")
         w("};")
         w("// the same for the fast form (near_check.cuh)")
-        w(f"__device__ const NearStep k{R}NearStep[{len(m['schedule'])}] = {{")
-        ne = ns = 0
-        for kind, gi in m["schedule"]:
-            n = _env_tests(m, gi) if kind == "env" else 0
-            ne, ns = ne + n, ns + (kind != "env")
-            w(f"    {{{0 if kind == 'env' else 1}, {gi}, {ne}, {ns}, {n if kind == 'env' else len(m['self_groups'][gi]['pairs'])}}},")
-        w("};")
         w(f"__device__ const NearPairBlock k{R}NearPair[{max(1, len(pblocks))}] = {{")
         for fa, fb, pf, n in pblocks or [(-1, -1, 0, 0)]:
             row, c, r = _rows(pair_rows[pf:pf + n])
@@ -490,9 +486,9 @@ def emit_cuda_checker(m: dict) -> str:
         w("};")
     w("")
 
-    def function(head, lines):
+    def function(head, lines, more=""):
         w("template <class Ctx>")
-        w(f"{head}(const float *__restrict__ q, Ctx &ctx)")
+        w(f"{head}(const float *__restrict__ q, Ctx &ctx{more})")
         w("{")
         for line in lines:
             w("    " + line)
@@ -503,18 +499,20 @@ def emit_cuda_checker(m: dict) -> str:
         """The fast form's answer, else the exact form's (on values the
         compiler cannot tell from new ones, so that it keeps none of the fast
         form's kinematics for them)."""
-        return ["const int a = near_check(q, ctx);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
+        return [f"StepMarks<{(len(m['schedule']) + 31) // 32}> marks;   // the steps that the exact form has to make",
+                "const int a = near_check(q, ctx, marks);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
                 "#pragma unroll", "for (int d = 0; d < kDof; d++) {", "    c[d] = q[d];",
-                '    asm volatile("" : "+f"(c[d]));', "}", f"if constexpr (Ctx::kInlineExact) return {exact}(c, ctx);",
+                '    asm volatile("" : "+f"(c[d]));', "}", f"if constexpr (Ctx::kInlineExact) return {exact}(c, ctx, marks);",
                 "Ctx own = ctx;   // the call must not force the caller's into memory",
-                f"const bool free = {exact}_call(c, own);", "ctx.work = own.work;", "return free;"]
+                f"const bool free = {exact}_call(c, own, marks);", "ctx.work = own.work;", "return free;"]
 
     if table:
         near_gates = near_ids
+        marks_type = f"StepMarks<{(len(m['schedule']) + 31) // 32}>"
         w(f"struct {R}Near {{")
         w(f"    static constexpr int kDof = {m['dof']}, kFrames = {len(m['joints'])}, kGates = {len(near_gates)}, "
           f"kWords = {(len(m['schedule']) + 31) // 32};")
-        for name_, type_, arr in (("steps", "NearStep", "NearStep"), ("env_groups", "GenEnvGroup", "EnvGroup"),
+        for name_, type_, arr in (("steps", "GenSched", "Sched"), ("env_groups", "GenEnvGroup", "EnvGroup"),
                                   ("leaf_blocks", "GenLeafBlock", "LeafBlock"), ("leaves", "float4", "Leaf"),
                                   ("self_groups", "GenSelfGroup", "SelfGroup"), ("pair_blocks", "NearPairBlock", "NearPair"),
                                   ("pairs", "LeafPair", "Pair")):
@@ -527,12 +525,14 @@ def emit_cuda_checker(m: dict) -> str:
         w("};")
         w("")
         for exact, lines in [("fkcc_exact", tcode.lines)] + ([("fkcc_validate_exact", code.lines)] if inline else []):
-            function(f"__device__ __forceinline__ bool {exact}", lines)
-            function(f"__device__ __noinline__ bool {exact}_call", [f"return {exact}(q, ctx);"])
-        function("__device__ __forceinline__ int near_check_leaves", _near_body(m, near_gates, LEAF_MARKS))
-        function("__device__ __forceinline__ int near_check_gates", _near_body(m, near_gates, ALWAYS))
+            function(f"__device__ __forceinline__ bool {exact}", lines, f", const {marks_type} &marks")
+            function(f"__device__ __noinline__ bool {exact}_call", [f"return {exact}(q, ctx, marks);"], f", const {marks_type} marks")
+        out_marks = f", {marks_type} &marks"
+        function("__device__ __forceinline__ int near_check_leaves", _near_body(m, near_gates, LEAF_MARKS), out_marks)
+        function("__device__ __forceinline__ int near_check_gates", _near_body(m, near_gates, ALWAYS), out_marks)
         function("__device__ __forceinline__ int near_check",
-                 ["if constexpr (Ctx::kLeafMarks) return near_check_leaves(q, ctx);", "else return near_check_gates(q, ctx);"])
+                 ["if constexpr (Ctx::kLeafMarks) return near_check_leaves(q, ctx, marks);",
+                  "else return near_check_gates(q, ctx, marks);"], out_marks)
     w("// Returns true when configuration q is collision-free.")
     function("__device__ __forceinline__ bool fkcc", fast_or("fkcc_exact") if table else code.lines)
     w("// The same verdicts for the stand-alone checker of single configurations.")
@@ -612,14 +612,16 @@ def _near_body(m, gate_ids, leaf_marks):
     code = _Code()
     fk = _FkGen(m, code)
     sp, w = m["spheres"], code.lines.append
+    steps = m["schedule"]
+    words = (len(steps) + 31) // 32
     w("const EnvGrid *grid = ctx.env.grid;")
+    w("#pragma unroll")
+    w(f"for (int w = 0; w < {words}; w++) marks.marked[w] = ~0u, marks.passed[w] = 0u;")
     w("if (!grid || !(grid->lo[0] <= grid->hi[0])) return kNearUnsure;")
     w(f"if (!({' + '.join(f'fabsf(q[{d}])' for d in range(m['dof']))} < 100.0f)) return kNearUnsure;")
     for jt in m["joints"]:
         if jt["type"] != "revolute":
             w(f"if (fabsf(q[{jt['q']}]) > 4.0f) return kNearUnsure;")
-    steps = m["schedule"]
-    words = (len(steps) + 31) // 32
     w("const NearView near = near_view(ctx);")
     w("unsigned " + ", ".join(f"m{k} = 0, p{k} = 0" for k in range(words)) + ";   // marked and passed steps")
     w("int extra = 0;   // FLOPs of the passed steps' leaf pairs")
@@ -701,11 +703,11 @@ def _near_body(m, gate_ids, leaf_marks):
     any_ = " | ".join(f"m{k}" for k in range(words))
     env_total = sum(_env_tests(m, gi) for kind, gi in steps if kind == "env")
     self_total = sum(kind != "env" for kind, _ in steps)
+    for k in range(words):
+        w(f"marks.marked[{k}] = m{k}, marks.passed[{k}] = p{k};")
     w(f"if ({any_}) {{")
     w("    if (ctx.stop()) return kNearFree;")
-    w(f"    const unsigned a = near_resolve<{R}Near>(NearCfg<kDof>{{{{{', '.join(f'q[{d}]' for d in range(m['dof']))}}}}},")
-    w(f"        NearMarks<{words}>{{{{{', '.join(f'm{k}' for k in range(words))}}}, {{{', '.join(f'p{k}' for k in range(words))}}}}}, "
-      "extra, grid, ctx.pad);")
+    w(f"    const unsigned a = near_resolve<{R}Near>(NearCfg<kDof>{{{{{', '.join(f'q[{d}]' for d in range(m['dof']))}}}}}, marks, extra, grid, ctx.pad);")
     w("    if ((a & 3u) == kNearHit) ctx.work += a >> 2;")
     w("    if ((a & 3u) != kNearFree) return (int)(a & 3u);")
     w("    extra = (int)a >> 2;")
