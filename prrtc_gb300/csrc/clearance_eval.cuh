@@ -17,8 +17,9 @@
 //    is applied to the joints that carry it directly, four joints at a time
 //    (no force tables, no sweep over joints without forces).
 // 4096 Panda paths of 64 waypoints on shelf scenes (k_path_cost_grad): 1.83 ms
-// with one thread per waypoint, 0.5 ms so; 1024 of them smoothed 44.6 -> 13.0 ms,
-// 32 Baxter paths 61.1 -> 4.1 ms.  Results differ from the one-thread form's by
+// with one thread per waypoint, 0.5 ms so; 1024 of them smoothed 44.6 -> 11.7 ms,
+// 32 Baxter paths 61.1 -> 3.7 ms (rows of pairs against the whole other frame
+// instead of parts of at most 6 spheres: 12.1 and 4.8 ms; parts of 4: 11.5 and 3.7).  Results differ from the one-thread form's by
 // 2e-10 (relative, all outputs), the error against float64 is the same 2.5e-8
 // (float32's own).
 #pragma once

@@ -62,8 +62,27 @@ inline float4 clr_ball(const std::vector<float4> &s)
     return make_float4((float)c[0], (float)c[1], (float)c[2], (float)(r * 1.00001 + 1e-5));
 }
 
-// The four-lane form's tables: each frame's leaves cut along their longest
-// extent into sets of at most 8, and the pairs of every two frames in rows.
+// Spheres cut along their longest extent into parts of at most `most`.
+inline std::vector<std::vector<float4>> clr_parts(std::vector<float4> s, int most)
+{
+    auto extent = [&](auto &&get) {
+        float lo = 1e30f, hi = -1e30f;
+        for (const float4 &p : s) lo = std::min(lo, get(p)), hi = std::max(hi, get(p));
+        return hi - lo;
+    };
+    const float ex = extent([](const float4 &p) { return p.x; }), ey = extent([](const float4 &p) { return p.y; }),
+                ez = extent([](const float4 &p) { return p.z; });
+    std::stable_sort(s.begin(), s.end(), [&](const float4 &a, const float4 &b) {
+        return ex >= ey && ex >= ez ? a.x < b.x : ey >= ez ? a.y < b.y : a.z < b.z;
+    });
+    const int n = (int)s.size(), parts = (n + most - 1) / most;
+    std::vector<std::vector<float4>> out;
+    for (int k = 0; k < parts; k++) out.emplace_back(s.begin() + n * k / parts, s.begin() + n * (k + 1) / parts);
+    return out;
+}
+
+// The four-lane form's tables: each frame's leaves in sets of at most 8, and the
+// pairs of every two frames in rows of one sphere against at most 6.
 inline void clr_sets(ClrHostModel &h)
 {
     h.chain.resize(h.joints.size());
@@ -71,23 +90,8 @@ inline void clr_sets(ClrHostModel &h)
     std::map<int, std::vector<float4>> frames;
     for (size_t i = 0; i < h.leaf.size(); i++) frames[h.leaf_joint[i]].push_back(h.leaf[i]);
     for (auto &[joint, leaves] : frames) {
-        auto extent = [&](auto &&get) {
-            float lo = 1e30f, hi = -1e30f;
-            for (const float4 &p : leaves) lo = std::min(lo, get(p)), hi = std::max(hi, get(p));
-            return hi - lo;
-        };
-        auto x = [](const float4 &p) { return p.x; };
-        auto y = [](const float4 &p) { return p.y; };
-        auto z = [](const float4 &p) { return p.z; };
-        const float ex = extent(x), ey = extent(y), ez = extent(z);
-        std::stable_sort(leaves.begin(), leaves.end(), [&](const float4 &a, const float4 &b) {
-            return ex >= ey && ex >= ez ? a.x < b.x : ey >= ez ? a.y < b.y : a.z < b.z;
-        });
-        const int n = (int)leaves.size(), sets = (n + 7) / 8;
-        for (int k = 0; k < sets; k++) {
-            const int from = n * k / sets, to = n * (k + 1) / sets;
-            const std::vector<float4> part(leaves.begin() + from, leaves.begin() + to);
-            h.leaf_sets.push_back(ClrLeafSet{clr_ball(part), joint, (int)h.set_leaves.size(), to - from, 0});
+        for (const std::vector<float4> &part : clr_parts(leaves, 8)) {
+            h.leaf_sets.push_back(ClrLeafSet{clr_ball(part), joint, (int)h.set_leaves.size(), (int)part.size(), 0});
             h.set_leaves.insert(h.set_leaves.end(), part.begin(), part.end());
         }
     }
@@ -111,12 +115,14 @@ inline void clr_sets(ClrHostModel &h)
             as.push_back(r.a);
             bs.insert(bs.end(), r.b.begin(), r.b.end());
         }
-        h.pair_sets.push_back(ClrPairSet{clr_ball(as), clr_ball(bs), frame.first, frame.second, (int)h.pair_rows.size(),
-                                         (int)rows.size()});
-        for (const Row &r : rows) {
-            h.pair_rows.push_back(ClrPairRow{r.a, clr_ball(r.b), (int)h.pair_spheres.size(), (int)r.b.size(), {0, 0}});
-            h.pair_spheres.insert(h.pair_spheres.end(), r.b.begin(), r.b.end());
-        }
+        h.pair_sets.push_back(ClrPairSet{clr_ball(as), clr_ball(bs), frame.first, frame.second, (int)h.pair_rows.size(), 0});
+        ClrPairSet &set = h.pair_sets.back();
+        for (const Row &r : rows)
+            for (const std::vector<float4> &part : clr_parts(r.b, 6)) {   // tighter balls around fewer spheres
+                h.pair_rows.push_back(ClrPairRow{r.a, clr_ball(part), (int)h.pair_spheres.size(), (int)part.size(), {0, 0}});
+                h.pair_spheres.insert(h.pair_spheres.end(), part.begin(), part.end());
+            }
+        set.n = (int)h.pair_rows.size() - set.first;
     }
 }
 
