@@ -14,6 +14,7 @@ context's device, used in place).  The shared library must have been built
 from __future__ import annotations
 
 import ctypes as C
+import operator
 from dataclasses import dataclass, field
 from pathlib import Path
 
@@ -216,11 +217,13 @@ def num_spheres(robot) -> int:
 class EnvHandle:
     def __init__(self, ctx: "Context", handle: C.c_void_p, env: Environment):
         self.ctx, self.handle, self.env = ctx, handle, env
+        self.address = handle.value
 
     def free(self):
         if self.handle:
             lib().prrtc_env_free(self.ctx.handle, self.handle)
             self.handle = None
+            del self.address
 
     def __del__(self):
         try:
@@ -344,6 +347,11 @@ class Context:
         return out
 
     def _env_table(self, envs, n_paths: int):
+        if isinstance(envs, (list, tuple)) and len(envs) == n_paths and set(map(type, envs)) == {EnvHandle}:
+            # uploaded environments: their addresses as one array (a ctypes
+            # array filled handle by handle took 0.9 ms for 4096 paths)
+            table = np.fromiter(map(_ADDRESS, envs), np.uint64, n_paths)
+            return table.ctypes.data_as(C.POINTER(C.c_void_p)), (envs, table)
         seen = {}   # one upload per distinct environment object
         hs = []
         for e in (envs if isinstance(envs, (list, tuple)) else [envs] * n_paths):
@@ -616,6 +624,7 @@ def _empty_like_device(t, shape, dtype: str):
     return torch.empty(shape, dtype=getattr(torch, dtype), device=t.device)
 
 
+_ADDRESS = operator.attrgetter("address")
 _QUERY_DT = _numpy_dtype(_Query)
 _DESC_DT = _numpy_dtype(EnvDesc)
 _RESULT_DT = _numpy_dtype(_Result)
