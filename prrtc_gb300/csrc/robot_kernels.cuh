@@ -36,13 +36,12 @@ __device__ __forceinline__ void add_work(unsigned long long *work, unsigned long
 }
 
 // Launch bounds of the stand-alone configuration checker, per robot: by
-// default at most 64 registers (128-thread blocks, 8 per SM), where the
-// straight-line checker spills a little but 32 resident warps per SM instead
-// of 16 hide its dependency waits better (2^20 random configurations: Panda
-// 1.23 vs 1.27 ms on the tabletop scene and 1.81 vs 1.97 ms on the shelf,
-// Baxter 3.70 ms against 4.50 ms unconstrained and 4.53 ms at 122 registers
-// on a shelf scene; Fetch, table form, 5.28 ms against 5.56 ms
-// unconstrained); a robot file may specialise it.
+// default at most 64 registers (128-thread blocks, 8 per SM): the marking code
+// spills a little but 32 resident warps per SM hide its waits better.  A
+// million random Panda configurations on a shelf scene: 826 us at 64
+// registers, 1142 at 80, 1212 at 96, 1040 at 128 (before the exact form was
+// cut down to marked steps and the sines were inlined; 782 us now).  A robot
+// file may specialise it.
 template <class Gen>
 struct ValidateLaunch {
     static constexpr int kMaxThreads = 128, kMinBlocks = 8;
@@ -66,8 +65,8 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
     // trip count) and meets at __syncwarp after every configuration: lanes
     // whose check ended early wait there instead of starting their next
     // configuration out of step with the rest.  Blocks are whole warps (128
-    // threads).  Baxter's table-form walk on 2^20 random configurations: 4.7
-    // instead of 17.2 ms, 13.7 instead of 3.7 lanes active per instruction.
+    // threads).  Without it Baxter's walk over 2^20 random configurations ran
+    // with 3.7 instead of 13.7 lanes active, 3.7 times as long.
     // spread: a warp takes 32 >> spread configurations at a time.
     const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> spread;
     for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> spread; w < n; w += stride) {

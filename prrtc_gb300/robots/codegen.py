@@ -6,11 +6,15 @@ Output, for each robot:
 * ``csrc/robots/<robot>_model.h``: the model as plain-C tables
   (``prrtc_joint_def`` ... from ``model_types.h``), read by the CPU oracle and
   by host code;
-* ``csrc/robots/<robot>_fkcc.cuh``: a straight-line CUDA forward-kinematics
-  and collision-check routine for one configuration per thread.  Joint
-  transforms are folded at generation time (zero and unit entries of the
-  fixed transforms vanish), every frame lives in registers, and the checker
-  visits the model's groups in the reference's order.  The per-leaf work runs
+* ``csrc/robots/<robot>_fkcc.cuh``: the CUDA checker for one configuration
+  per thread, in two forms.  The fast form (``near_check_*``) marks, in
+  straight-line code, the groups that can possibly collide (bounds from the
+  environment's clearance grid and from gate distances); only marked groups
+  are walked, and where the answer is within rounding of contact the exact
+  form decides.  The exact form visits the model's groups in the reference's
+  order.  Joint transforms are folded at generation time (zero and unit
+  entries of the fixed transforms vanish).  Also here: the joint rows of the
+  clearance's kinematics (``clr_rows``).  The per-leaf work runs
   in three small shared routines supplied by the caller (``Ctx``), so code
   size stays proportional to the number of groups, not of sphere pairs:
 
@@ -34,17 +38,17 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE.parent / "csrc" / "robots"
 ROBOTS = ("sphere", "panda", "fetch", "baxter")
 INLINE_LEAVES = 6   # leaf blocks up to this size are emitted as straight-line tests
-# Robots whose checker is emitted in table form: every frame computed first,
+# Robots whose exact form is emitted in table form: every frame computed first,
 # then one loop over the group schedule (run_schedule in device_common.cuh).
 # Baxter's 388 groups as straight-line code overflow the instruction cache
 # (its planner kernel stalled on instruction fetch 33 times per issue).
 TABLE_ROBOTS = ("panda", "fetch", "baxter")
-# Robots that also get the straight-line form, as fkcc_validate: Panda's
-# stand-alone checker runs 6 % faster with it than with the table form (2^20
-# random configurations, tabletop scene: 1.24 vs 1.32 ms).  Fetch's runs 2 %
-# faster in table form at 64 registers (mixed scene: 5.28 vs 5.38 ms) and
-# Baxter's straight-line form does not fit the instruction cache, so both
-# use the table form for single configurations too.
+# Robots that also get the straight-line exact form, as fkcc_validate_exact.
+# Which form decides single configurations within rounding of contact is part
+# of their verdicts (the two are contracted differently), so it stays as it
+# was chosen when the exact form made every check: 2^20 random configurations,
+# Panda straight-line 1.24 ms, table 1.32; Fetch 5.38 against 5.28; Baxter's
+# straight-line form does not fit the instruction cache.
 INLINE_VALIDATE = ("sphere", "panda")
 
 
