@@ -60,3 +60,27 @@ def test_counts_around_each_spread(robot, ctx, plain):
     want = plain(robot, env, q)
     for n in sorted({1, 31, 33} | {(lanes >> s) + d for s in range(6) for d in (-1, 0, 1)}):
         assert (ctx.validate_configs(robot, env, q[:n]) == want[:n]).all(), n
+
+
+@pytest.mark.parametrize("robot,waypoints,paths", [("panda", 32, 3), ("panda", 33, 3), ("panda", 65, 400), ("fetch", 129, 2),
+                                                   ("baxter", 256, 1)])
+def test_smoothing_at_its_block_sizes(robot, waypoints, paths, ctx, plain):
+    """128 and 256 threads, waypoints beyond one pass, the largest environment
+    beside the longest path: a path is returned as it came or free edge by edge,
+    and its cost before is path_cost_grad's (both sums of the same FP64 terms,
+    rounded to float32 at the end, there per waypoint)."""
+    from prrtc_gb300 import SmoothSettings
+    from prrtc_gb300.env import Environment
+    rng = np.random.default_rng(waypoints)
+    far = np.column_stack([rng.uniform(1.5, 2.5, (2815, 3)), rng.uniform(0.005, 0.02, 2815)]).astype(np.float32)
+    env = ctx.upload_env(Environment(spheres=[[0.6, 0.0, 0.9, 0.1], *far]))
+    ends = _configs(robot, 2 * paths, 3).reshape(paths, 2, 1, -1)
+    t = np.linspace(0.0, 1.0, waypoints, dtype=np.float32)[None, :, None]
+    q = (ends[:, 0] + t * (0.1 * (ends[:, 1] - ends[:, 0]))).astype(np.float32)
+    cost, _ = ctx.path_cost_grad(robot, env, q)
+    out, acc, before, after = ctx.smooth_paths(robot, env, q, SmoothSettings(steps=2, granularity=5))
+    total = cost.astype(np.float64).sum(1)
+    assert (np.abs(before - total) <= 2.0 ** -22 * total + 1e-12).all()
+    assert (out[acc == 0] == q[acc == 0]).all() and np.isfinite(after).all()
+    for p in np.flatnonzero(acc):
+        assert ctx.validate_edges(robot, env, out[p, :-1], out[p, 1:], 5).all()
