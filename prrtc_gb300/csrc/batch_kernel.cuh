@@ -622,7 +622,11 @@ __global__ void __launch_bounds__(128, 3) k_rrtc_batch(const BatchParams P)
                 scan_from++;
             }
             const unsigned s0 = scan_from;
-            const bool pending = vload(&C->admit_next) < P.num_queries;
+            // (other warps move the queue on meanwhile: one lane's reading for all,
+            // as whole-warp instructions below depend on it)
+            int pending = 0;
+            if (lane == 0) pending = vload(&C->admit_next) < P.num_queries;
+            pending = __shfl_sync(FULL, pending, 0);
             const unsigned long long now = global_ns();
             for (int base = 0; base < P.num_slots && found < 0 && rec < 0; base += 32) {
                 const int s = (int)((s0 + (unsigned)(base + lane)) % (unsigned)P.num_slots);
