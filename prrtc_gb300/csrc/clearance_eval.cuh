@@ -259,54 +259,56 @@ __device__ double eval(EvalScratch<Gen::kFrames - 1> &S, const ClrModel &M, cons
     // their leaves, four at a time
     const EnvGrid *grid = e.grid && e.grid->lo[0] <= e.grid->hi[0] ? e.grid : nullptr;
     const float reach = mf + 2.0f * kScreen, keep = -kScreen - mf;
-    unsigned sets = 0;
-    for (int s0 = 0; s0 < M.n_leaf_sets; s0 += 4) {
-        const int s = s0 + l;
-        bool near = false;
-        if (run && s < M.n_leaf_sets) {
-            const ClrLeafSet L = M.leaf_sets[s];
-            near = env_near(grid, place_hi(S.hi, L.joint, L.ball), L.ball.w + reach);
-        }
-        sets |= (__ballot_sync(FULL, near) >> base & 15u) << s0;
-    }
-    int i = 0, n = 0, joint = -1;
-    while (true) {
-        if (i >= n && sets) {
-            const ClrLeafSet L = M.leaf_sets[__ffs(sets) - 1];
-            sets &= sets - 1;
-            i = L.first;
-            n = L.first + L.n;
-            joint = L.joint;
-        }
-        if (!__any_sync(FULL, i < n)) break;
-        bool have = false;
-        double3 g = d3(0.0, 0.0, 0.0), c = g;
-        if (i + l < n) {
-            const float4 s = M.set_leaves[i + l];
-            const float3 cf = place_hi(S.hi, joint, s);
-            if (env_near(grid, cf, s.w + reach)) {
-                bool placed = false;
-                auto centre = [&]() {
-                    if (!placed) c = place_dd(S, joint, s);
-                    placed = true;
-                    return c;
-                };
-                const int cell = grid ? grid_cell(*grid, cf.x, cf.y, cf.z) : -1;
-                const int t = __float2int_ru((s.w + reach) * kGridUnit);
-                unsigned listed = cell >= 0 && t <= 255 ? listed_below(*grid, cell, t) : 1u << kGridListed;
-                if (listed >> kGridListed) {
-                    for (int k = 0; k < e.n.obstacles(); k++)
-                        obstacle_term(e.rec, e.n, k, cf, s.w, keep, m, centre, &cost, &g);
-                } else {
-                    const uint8_t *num = reinterpret_cast<const uint8_t *>(grid->list + 2 * cell + 1);
-                    for (; listed; listed &= listed - 1)
-                        obstacle_term(e.rec, e.n, __ldg(num + __ffs(listed) - 1), cf, s.w, keep, m, centre, &cost, &g);
-                }
-                have = joint >= 0 && (g.x != 0.0 || g.y != 0.0 || g.z != 0.0);
+    for (int p0 = 0; p0 < M.n_leaf_sets; p0 += 32) {   // a bit per set
+        unsigned sets = 0;
+        for (int s0 = 0; s0 < 32 && p0 + s0 < M.n_leaf_sets; s0 += 4) {
+            const int s = p0 + s0 + l;
+            bool near = false;
+            if (run && s < M.n_leaf_sets) {
+                const ClrLeafSet L = M.leaf_sets[s];
+                near = env_near(grid, place_hi(S.hi, L.joint, L.ball), L.ball.w + reach);
             }
+            sets |= (__ballot_sync(FULL, near) >> base & 15u) << s0;
         }
-        apply(have, c, g, joint >= 0 ? M.chain[joint] : 0u);
-        i += 4;
+        int i = 0, n = 0, joint = -1;
+        while (true) {
+            if (i >= n && sets) {
+                const ClrLeafSet L = M.leaf_sets[p0 + __ffs(sets) - 1];
+                sets &= sets - 1;
+                i = L.first;
+                n = L.first + L.n;
+                joint = L.joint;
+            }
+            if (!__any_sync(FULL, i < n)) break;
+            bool have = false;
+            double3 g = d3(0.0, 0.0, 0.0), c = g;
+            if (i + l < n) {
+                const float4 s = M.set_leaves[i + l];
+                const float3 cf = place_hi(S.hi, joint, s);
+                if (env_near(grid, cf, s.w + reach)) {
+                    bool placed = false;
+                    auto centre = [&]() {
+                        if (!placed) c = place_dd(S, joint, s);
+                        placed = true;
+                        return c;
+                    };
+                    const int cell = grid ? grid_cell(*grid, cf.x, cf.y, cf.z) : -1;
+                    const int t = __float2int_ru((s.w + reach) * kGridUnit);
+                    unsigned listed = cell >= 0 && t <= 255 ? listed_below(*grid, cell, t) : 1u << kGridListed;
+                    if (listed >> kGridListed) {
+                        for (int k = 0; k < e.n.obstacles(); k++)
+                            obstacle_term(e.rec, e.n, k, cf, s.w, keep, m, centre, &cost, &g);
+                    } else {
+                        const uint8_t *num = reinterpret_cast<const uint8_t *>(grid->list + 2 * cell + 1);
+                        for (; listed; listed &= listed - 1)
+                            obstacle_term(e.rec, e.n, __ldg(num + __ffs(listed) - 1), cf, s.w, keep, m, centre, &cost, &g);
+                    }
+                    have = joint >= 0 && (g.x != 0.0 || g.y != 0.0 || g.z != 0.0);
+                }
+            }
+            apply(have, c, g, joint >= 0 ? M.chain[joint] : 0u);
+            i += 4;
+        }
     }
 
     // sphere pairs: frame pairs whose balls come near, then their rows
