@@ -270,33 +270,24 @@ CLR_FN float3 place(const float (*T)[12], int j, float4 p)
 
 // ---- one configuration -------------------------------------------------
 
-// Every obstacle against leaf sphere l on joint j: float32 screen at cf,
-// float64 terms at the exact centre.  Adds the cost, returns dC/dc.
-static __host__ __device__ double3 env_force(const ClrEnv e, const double (*T)[12], int j, float4 l, float3 cf,
-                                             double m, double *cost)
+// Every obstacle against a leaf sphere of radius r: float32 screen at cf,
+// float64 terms at centre() (asked for when a term is kept).  Adds the cost to
+// *cost and dC/dc to *g.
+template <class Centre>
+CLR_FN void env_terms(const ClrEnv &e, float3 cf, float r, float keep, double m, Centre &&centre, double *cost, double3 *g)
 {
-    double3 g = d3(0.0, 0.0, 0.0), c = g;
-    bool have = false;
-    const float r = l.w, keep = -kScreen - (float)m;   // kept when sd_f < m + kScreen
-    auto centre = [&]() {
-        if (!have) {
-            c = place(T, j, l);
-            have = true;
-        }
-        return c;
-    };
     const float4 *p = e.rec;
     for (int i = 0; i < e.n.ns; i++) {
         const float4 s = p[i];
         if (-sd_point_f(sub(cf, f3(s.x, s.y, s.z)), r + s.w) > keep)
-            point_term(sub(centre(), d3(s.x, s.y, s.z)), (double)r + s.w, m, cost, &g);
+            point_term(sub(centre(), d3(s.x, s.y, s.z)), (double)r + s.w, m, cost, g);
     }
     p += e.n.ns;
     for (int k = 0; k < 2; k++) {
         const int n = k ? e.n.nzc : e.n.nc;
         for (int i = 0; i < n; i++) {
             const float4 a = p[2 * i], v = p[2 * i + 1];   // (x1, y1, z1, r) (xv, yv, zv, 1/|v|^2)
-            if (-sd_capsule_f(cf, r, a, v, k) > keep) capsule_term(centre(), r, a, v, k, m, cost, &g);
+            if (-sd_capsule_f(cf, r, a, v, k) > keep) capsule_term(centre(), r, a, v, k, m, cost, g);
         }
         p += 2 * n;
     }
@@ -308,10 +299,26 @@ static __host__ __device__ double3 env_force(const ClrEnv e, const double (*T)[1
             const float3 a1 = f3(c1.x, c1.y, k ? 0.0f : c1.z), a2 = f3(c2.x, c2.y, k ? 0.0f : c2.z),
                          a3 = k ? f3(0.0f, 0.0f, 1.0f) : f3(c3.x, c3.y, c3.z), ce = f3(c0.x, c0.y, c0.z),
                          h = f3(c0.w, c1.w, c2.w);
-            if (-sd_box_f(cf, r, ce, a1, a2, a3, h) > keep) box_term(centre(), r, ce, a1, a2, a3, h, m, cost, &g);
+            if (-sd_box_f(cf, r, ce, a1, a2, a3, h) > keep) box_term(centre(), r, ce, a1, a2, a3, h, m, cost, g);
         }
         p += 4 * n;
     }
+}
+
+// Every obstacle against leaf sphere l on joint j, at cf in float32.
+static __host__ __device__ double3 env_force(const ClrEnv e, const double (*T)[12], int j, float4 l, float3 cf,
+                                             double m, double *cost)
+{
+    double3 g = d3(0.0, 0.0, 0.0), c = g;
+    bool have = false;
+    auto centre = [&]() {
+        if (!have) {
+            c = place(T, j, l);
+            have = true;
+        }
+        return c;
+    };
+    env_terms(e, cf, l.w, -kScreen - (float)m, m, centre, cost, &g);   // kept when sd_f < m + kScreen
     return g;
 }
 

@@ -296,8 +296,7 @@ __device__ double eval(EvalScratch<Gen::kFrames - 1> &S, const ClrModel &M, cons
                     const int t = __float2int_ru((s.w + reach) * kGridUnit);
                     unsigned listed = cell >= 0 && t <= 255 ? listed_below(*grid, cell, t) : 1u << kGridListed;
                     if (listed >> kGridListed) {
-                        for (int k = 0; k < e.n.obstacles(); k++)
-                            obstacle_term(e.rec, e.n, k, cf, s.w, keep, m, centre, &cost, &g);
+                        env_terms(e, cf, s.w, keep, m, centre, &cost, &g);
                     } else {
                         const uint8_t *num = reinterpret_cast<const uint8_t *>(grid->list + 2 * cell + 1);
                         for (; listed; listed &= listed - 1)
