@@ -211,10 +211,12 @@ __device__ __forceinline__ bool sample_group(const BatchParams &P, const WarpScr
 template <class Ctx>
 __device__ __forceinline__ Ctx make_ctx(const EnvView &view, float pad, volatile int *stop, float4 *frames)
 {
-    if constexpr (Ctx::kSharedFrames)
-        return Ctx{PlanCheckCtx{{view, pad, stop}}, frames};
-    else
-        return Ctx{{view, pad, stop}};
+    Ctx ctx{};
+    ctx.env = view;
+    ctx.pad = pad;
+    ctx.stop_flag = stop;
+    if constexpr (Ctx::kSharedFrames) ctx.frames = frames;
+    return ctx;
 }
 
 // Whole warp: check the g points of the edge in W (from + k * step),
@@ -807,14 +809,20 @@ __global__ void __launch_bounds__(128, 3) k_rrtc_batch(const BatchParams P)
             staged_grid = Qd.grid;
         }
         if (new_query) {
-            if (lane == 0) W.view = EnvView{envp, Qd.env_n, Qd.grid ? &W.grid : nullptr};
+            // (a batch's own grids are built without asking whether the obstacles can have one)
+            if (lane == 0)
+                W.view = EnvView{envp, Qd.env_n, Qd.grid && W.grid.lo[0] <= W.grid.hi[0] ? &W.grid : nullptr};
             __syncwarp();
         }
         // every point of an edge through the robot's checker, frames where P says
         auto validate = [&]() {
-            return P.shared_frames
-                       ? warp_validate<Gen, SharedCheckCtx>(W, W_frames + lane, P.granularity, P.edge_order, P.pad, C->work)
-                       : warp_validate<Gen, PlanCheckCtx>(W, nullptr, P.granularity, P.edge_order, P.pad, C->work);
+            auto with = [&](auto local, auto shared) {
+                return P.shared_frames ? warp_validate<Gen, decltype(shared)>(W, W_frames + lane, P.granularity,
+                                                                              P.edge_order, P.pad, C->work)
+                                       : warp_validate<Gen, decltype(local)>(W, nullptr, P.granularity, P.edge_order,
+                                                                             P.pad, C->work);
+            };
+            return W.view.grid ? with(PlanCheckCtx{}, SharedCheckCtx{}) : with(EveryCheckCtx{}, SharedEveryCheckCtx{});
         };
         float *nodes_s = P.nodes + (size_t)slot * 2 * D * P.cap;
         int *par_s = P.parents + (size_t)slot * 2 * P.cap;

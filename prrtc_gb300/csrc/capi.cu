@@ -291,9 +291,14 @@ prrtc_status prrtc_env_upload(prrtc_ctx *ctx, const prrtc_env_desc *d, prrtc_env
     if (!e->host.empty()) {
         cudaSetDevice(c->device);
         const size_t rec_bytes = e->host.size() * sizeof(float4);
-        // room for the grid if there is any (without it the checker tests every obstacle)
-        bool grid = cudaMalloc(&e->dev, rec_bytes + env_grid_bytes(kEnvCells)) == cudaSuccess;
-        if (!grid && (cudaGetLastError(), cudaMalloc(&e->dev, rec_bytes) != cudaSuccess)) {
+        // room for the grid if these obstacles can have one and there is any
+        // (without it the checker tests every obstacle)
+        bool grid = env_grid_usable(e->host.data(), e->counts);
+        if (grid && cudaMalloc(&e->dev, rec_bytes + env_grid_bytes(kEnvCells)) != cudaSuccess) {
+            cudaGetLastError();
+            grid = false;
+        }
+        if (!grid && cudaMalloc(&e->dev, rec_bytes) != cudaSuccess) {
             cudaGetLastError();
             delete e;
             return c->fail(PRRTC_ENOMEM, "env_upload: cudaMalloc failed");

@@ -4,6 +4,7 @@
 
 #include "clearance_device.cuh"
 #include "clearance_eval.cuh"
+#include "near_check.cuh"
 #include "planner_device.cuh"
 
 namespace prrtc {
@@ -40,6 +41,17 @@ __host__ __device__ constexpr size_t smooth_eval_offset(int records, int waypoin
     return (records * sizeof(float4) + 2 * sizeof(float) * waypoints * Gen::kDof + 15) & ~(size_t)15;
 }
 
+// The check of a point in an environment without a grid, as a called function
+// (EveryCheckCtx, device_common.cuh).
+template <class Gen>
+__device__ __noinline__ bool every_test(const NearCfg<Gen::kDof> c, const EnvView env, volatile int *stop)
+{
+    EveryCheckCtx ctx{};
+    ctx.env = env;
+    ctx.stop_flag = stop;
+    return Gen::fkcc(c.q, ctx);
+}
+
 template <class Gen>
 __global__ void __launch_bounds__(256) k_smooth_paths(const ClrLaunch P)
 {
@@ -64,6 +76,10 @@ __global__ void __launch_bounds__(256) k_smooth_paths(const ClrLaunch P)
     const ClrEnv e{s_dyn, pe.n, gr};
     const ClrSmooth s = P.s;
     CheckCtx ctx{EnvView{e.rec, e.n, gr}, 0.0f, &s_bad};
+    auto is_free = [&](const NearCfg<D> &c) {
+        ctx.work = 0;
+        return gr ? Gen::fkcc(c.q, ctx) : every_test<Gen>(c, ctx.env, &s_bad);
+    };
     const int group = threadIdx.x >> 2, groups = blockDim.x >> 2, l = threadIdx.x & 3;
     // every waypoint's cost (returned summed over this thread's) and gradient
     auto evaluate = [&](auto &&store) {
@@ -95,15 +111,14 @@ __global__ void __launch_bounds__(256) k_smooth_paths(const ClrLaunch P)
         for (int idx = threadIdx.x; idx < span * gs; idx += blockDim.x) {
             if (*(volatile int *)&s_bad) break;
             const int m = idx / gs, k = idx - m * gs + 1;
-            float cfg[D];
+            NearCfg<D> cfg;
 #pragma unroll
             for (int d = 0; d < D; d++) {
                 const float delta = qb[d] - qa[d];
                 const float a = qa[d] + ((float)m / (float)span) * delta, b = qa[d] + ((float)(m + 1) / (float)span) * delta;
-                cfg[d] = __fadd_rn(a, __fmul_rn((float)k, __fdiv_rn(__fsub_rn(b, a), (float)gs)));
+                cfg.q[d] = __fadd_rn(a, __fmul_rn((float)k, __fdiv_rn(__fsub_rn(b, a), (float)gs)));
             }
-            ctx.work = 0;
-            if (!Gen::fkcc(cfg, ctx)) s_bad = 1;
+            if (!is_free(cfg)) s_bad = 1;
         }
         __syncthreads();
         if (s_bad == 0)
@@ -145,11 +160,10 @@ __global__ void __launch_bounds__(256) k_smooth_paths(const ClrLaunch P)
         if (*(volatile int *)&s_bad) break;
         const int ed = idx / s.granularity, k = idx - ed * s.granularity + 1;
         const float *a = s_q + ed * D, *b = a + D;
-        float cfg[D];
+        NearCfg<D> cfg;
 #pragma unroll
-        for (int d = 0; d < D; d++) cfg[d] = __fadd_rn(a[d], __fmul_rn((float)k, __fdiv_rn(__fsub_rn(b[d], a[d]), fg)));
-        ctx.work = 0;
-        if (!Gen::fkcc(cfg, ctx)) s_bad = 1;
+        for (int d = 0; d < D; d++) cfg.q[d] = __fadd_rn(a[d], __fmul_rn((float)k, __fdiv_rn(__fsub_rn(b[d], a[d]), fg)));
+        if (!is_free(cfg)) s_bad = 1;
     }
     __syncthreads();
     const bool ok = s_bad == 0;

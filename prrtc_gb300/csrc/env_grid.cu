@@ -29,7 +29,7 @@ __device__ __forceinline__ float clamp01(float v) { return fmaxf(fminf(v, 1.0f),
 // the box around obstacle k, and whether every value of it is one the bounds
 // hold for: at most kGridReach in size, axes no longer than 2, a capsule's
 // rdv the inverse square of its length (or the length zero)
-__device__ bool obstacle_box(const float4 *rec, const EnvCounts &n, int k, Box &b)
+__host__ __device__ bool obstacle_box(const float4 *rec, const EnvCounts &n, int k, Box &b)
 {
     auto small = [](float v, float most) { return fabsf(v) <= most; };   // false for NaN
     float c[3], e[3];
@@ -264,6 +264,14 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
 
 // (the lists, 16-byte entries, follow the header and a multiple of 16 bytes)
 static_assert(sizeof(EnvGrid) % 16 == 0, "the lists behind the header are 16-byte entries");
+bool env_grid_usable(const float4 *rec, const EnvCounts &n)
+{
+    Box b;
+    bool ok = n.obstacles() >= 1 && n.obstacles() <= kGridMaxObstacles;
+    for (int k = 0; ok && k < n.obstacles(); k++) ok = obstacle_box(rec, n, k, b);
+    return ok;
+}
+
 size_t env_grid_bytes(int cells) { return sizeof(EnvGrid) + (size_t)cells * 33; }
 
 cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st)

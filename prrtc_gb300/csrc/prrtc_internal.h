@@ -209,6 +209,7 @@ struct GoalQuery {
 // cells (a multiple of 16), and the launch that builds those of the n
 // descriptors that ask for it (device array `many`, or the single `one`).
 size_t env_grid_bytes(int cells);
+bool env_grid_usable(const float4 *rec, const EnvCounts &n);   // (host records) may there be a grid?
 cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st);
 
 struct ClrLaunch;   // clearance_device.cuh

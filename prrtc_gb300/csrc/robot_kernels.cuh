@@ -2,6 +2,8 @@
 // robot's generated checker; GEN names the generated namespace.
 #pragma once
 
+#include <algorithm>
+
 #include "clearance_kernel.cuh"
 #include "device_common.cuh"
 #include "planner_device.cuh"
@@ -136,9 +138,59 @@ __global__ void __launch_bounds__(128, 6) k_validate_edges(const float4 *__restr
     add_work(work, flops, cfgs);
 }
 
+// Edges in an environment without a grid (EveryTest): a block per edge
+// (grid-stride), thread t checks points k = t + 1, t + 1 + blockDim, ...
+// Every point takes about as long, so that the block's warps hardly wait for
+// one another, and the points' loop holds nothing but the check.  MinBlocks >
+// 0 builds it for that many resident 128-thread blocks per SM: 8 (at most 64
+// registers) is faster for 128-point edges (2^14 Panda edges on a shelf
+// scene 1.79 against 1.91 ms) and slower for the 32-thread blocks of short
+// edges, which keep the unconstrained build (0).
+template <class Gen, int MinBlocks>
+__global__ void __launch_bounds__(128, MinBlocks) k_validate_edges_every(const float4 *__restrict__ env, EnvCounts nc,
+                                                        const float *__restrict__ a, const float *__restrict__ b,
+                                                        int64_t n, int g, uint8_t *__restrict__ out,
+                                                        unsigned long long *work)
+{
+    unsigned long long flops = 0, cfgs = 0;
+    constexpr int D = Gen::kDof;
+    extern __shared__ float4 s_env[];
+    __shared__ float s_a[D], s_step[D];
+    __shared__ int s_bad;
+    __shared__ unsigned long long s_bar;
+    stage_env_bulk(s_env, env, nc.records(), &s_bar);
+    EveryCheckCtx ctx{};
+    ctx.env = EnvView{s_env, nc};
+    ctx.stop_flag = &s_bad;
+    const float fg = (float)g;
+    for (int64_t e = blockIdx.x; e < n; e += gridDim.x) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_bad = 0;
+        if (threadIdx.x < D) {
+            const float av = __ldg(a + e * D + threadIdx.x);
+            s_a[threadIdx.x] = av;
+            s_step[threadIdx.x] = __fdiv_rn(__fsub_rn(__ldg(b + e * D + threadIdx.x), av), fg);
+        }
+        __syncthreads();
+        for (int k = threadIdx.x + 1; k <= g; k += blockDim.x) {
+            if (s_bad) break;
+            float cfg[D];
+#pragma unroll
+            for (int d = 0; d < D; d++) cfg[d] = __fadd_rn(s_a[d], __fmul_rn((float)k, s_step[d]));
+            ctx.work = 0;
+            if (!Gen::fkcc(cfg, ctx)) s_bad = 1;
+            flops += ctx.work + Gen::kFkFlops;
+            cfgs++;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) out[e] = s_bad ? 0 : 1;
+    }
+    add_work(work, flops, cfgs);
+}
+
 // Goal-region candidates: flags[t] = 1 when candidate t (goal_candidate)
 // puts the chosen sphere's centre in the box and the checker finds it free.
-template <class Gen>
+template <class Gen, class Ctx>
 __global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ env, EnvCounts nc,
                                                     const EnvGrid *grid, const GoalQuery g, uint8_t *__restrict__ flags)
 {
@@ -147,7 +199,8 @@ __global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ e
     __shared__ EnvGrid s_grid;
     const EnvGrid *gr = stage_grid(&s_grid, grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
-    SingleCheckCtx ctx{{{s_env, nc, gr}, 0.0f, nullptr}};
+    Ctx ctx{};
+    ctx.env = EnvView{s_env, nc, gr};
     // warp-uniform trip count, lanes meeting after every candidate (as in k_validate_configs)
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long tw = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); tw < g.tries; tw += stride) {
@@ -220,7 +273,7 @@ __global__ void __launch_bounds__(32) k_fk_spheres(const float *__restrict__ q, 
 //    before failing, pRRTC.cu:451-454,535-537), the traceback is bounded by
 //    the path buffer, and the DD CAS loops are bounded;
 //  * an optional device time budget ends the search with solved = -2.
-template <class Gen>
+template <class Gen, class Ctx>
 __global__ void __launch_bounds__(256) k_rrtc_plain(const PlainParams P)
 {
     constexpr int D = Gen::kDof;
@@ -244,7 +297,10 @@ __global__ void __launch_bounds__(256) k_rrtc_plain(const PlainParams P)
     __shared__ EnvGrid s_grid;
     const EnvGrid *gr = stage_grid(&s_grid, P.grid, s_env, threadIdx.x, blockDim.x);
     stage_env_bulk(s_env, P.env, P.env_n.records(), &s_bar);   // synchronises the block
-    CheckCtx ctx{{s_env, P.env_n, gr}, P.pad, &s_bad};
+    Ctx ctx{};
+    ctx.env = EnvView{s_env, P.env_n, gr};
+    ctx.pad = P.pad;
+    ctx.stop_flag = &s_bad;
     const float fg = (float)P.granularity;
     const unsigned long long t0 = P.budget_ns ? global_ns() : 0ull;
     int iter = 0;
@@ -449,7 +505,10 @@ struct RobotKernels {
         int spread = 0;
         while (spread < 5 && (n << (spread + 1)) <= (int64_t)le.sms * 8 * 32) spread++;
         const int blocks = grid_for(n << spread, threads, le.sms, 16);
-        if (spread >= 3)   // at most 4 configurations to a warp
+        if (!le.grid)
+            k_validate_configs<Gen, EveryCheckCtx><<<blocks, threads, smem, st>>>(le.rec, le.counts, nullptr, q, n, out,
+                                                                                  le.work, spread);
+        else if (spread >= 3)   // at most 4 configurations to a warp
             k_validate_configs<Gen, SingleCheckCtx><<<blocks, threads, smem, st>>>(le.rec, le.counts, le.grid, q, n, out,
                                                                                    le.work, spread);
         else
@@ -462,10 +521,20 @@ struct RobotKernels {
     {
         if (n <= 0) return cudaSuccess;
         const size_t smem = (size_t)le.counts.records() * sizeof(float4);
+        const int chunks = (g + 31) / 32;
+        if (!le.grid) {
+            const int threads = 32 * std::min(chunks, 4);
+            const int blocks = (int)std::min<int64_t>(n, (int64_t)le.sms * (2048 / threads));
+            if (threads == 128)
+                k_validate_edges_every<Gen, 8><<<blocks, threads, smem, st>>>(le.rec, le.counts, a, b, n, g, out, le.work);
+            else
+                k_validate_edges_every<Gen, 0><<<blocks, threads, smem, st>>>(le.rec, le.counts, a, b, n, g, out, le.work);
+            return cudaGetLastError();
+        }
         const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
         if (e != cudaSuccess) return e;
-        k_validate_edges<Gen><<<grid_for(n * ((g + 31) / 32) * 32, 128, le.sms, 16), 128, smem, st>>>(
-            le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
+        k_validate_edges<Gen><<<grid_for(n * chunks * 32, 128, le.sms, 16), 128, smem, st>>>(le.rec, le.counts, le.grid, a, b,
+                                                                                           n, g, out, le.work);
         return cudaGetLastError();
     }
     static cudaError_t fk_spheres(const float *q, int64_t n, float *out, int sms, cudaStream_t st)
@@ -482,7 +551,10 @@ struct RobotKernels {
     static cudaError_t solve_plain(const PlainParams &P, int threads, cudaStream_t st)
     {
         const size_t smem = (size_t)P.env_n.records() * sizeof(float4);
-        k_rrtc_plain<Gen><<<P.num_new_configs, threads, smem, st>>>(P);
+        if (P.grid)
+            k_rrtc_plain<Gen, CheckCtx><<<P.num_new_configs, threads, smem, st>>>(P);
+        else
+            k_rrtc_plain<Gen, EveryCheckCtx><<<P.num_new_configs, threads, smem, st>>>(P);
         return cudaGetLastError();
     }
     static cudaError_t solve_batch(const BatchParams &P, int blocks, int wpb, cudaStream_t st)
@@ -513,7 +585,11 @@ struct RobotKernels {
     {
         if (g.tries <= 0) return cudaSuccess;
         const size_t smem = (size_t)le.counts.records() * sizeof(float4);
-        k_goal_flags<Gen><<<grid_for(g.tries, 128, le.sms, 16), 128, smem, st>>>(le.rec, le.counts, le.grid, g, flags);
+        const int blocks = grid_for(g.tries, 128, le.sms, 16);
+        if (le.grid)
+            k_goal_flags<Gen, SingleCheckCtx><<<blocks, 128, smem, st>>>(le.rec, le.counts, le.grid, g, flags);
+        else
+            k_goal_flags<Gen, EveryCheckCtx><<<blocks, 128, smem, st>>>(le.rec, le.counts, nullptr, g, flags);
         return cudaGetLastError();
     }
     static cudaError_t path_cost_grad(const ClrModel &M, const ClrEnv *envs, int64_t rows, int waypoints, const float *q,

@@ -445,7 +445,9 @@ def emit_cuda_checker(m: dict) -> str:
         for kind, gi in m["schedule"]:
             n = _env_tests(m, gi) if kind == "env" else len(m["self_groups"][gi]["pairs"])
             ne, ns = (ne + n, ns) if kind == "env" else (ne, ns + 1)
-            w(f"    {{{0 if kind == 'env' else 1}, {gi}, {ne}, {ns}, {n}}},")
+            row = (gi if kind == "env" else -1 - gi, ne, ns, n)
+            assert max(map(abs, row)) < 1 << 15, "GenSched's fields are 16 bits wide"
+            w("    {%d, %d, %d, %d}," % row)
         w("};")
         lblocks, eg_rows = [], []
         for gi, g in enumerate(m["env_groups"]):
@@ -490,8 +492,8 @@ def emit_cuda_checker(m: dict) -> str:
         w("};")
     w("")
 
-    def function(head, lines, more=""):
-        w("template <class Ctx>")
+    def function(head, lines, more="", types="class Ctx"):
+        w(f"template <{types}>")
         w(f"{head}(const float *__restrict__ q, Ctx &ctx{more})")
         w("{")
         for line in lines:
@@ -503,12 +505,16 @@ def emit_cuda_checker(m: dict) -> str:
         """The fast form's answer, else the exact form's (on values the
         compiler cannot tell from new ones, so that it keeps none of the fast
         form's kinematics for them)."""
-        return [f"StepMarks<{(len(m['schedule']) + 31) // 32}> marks;   // the steps that the exact form has to make",
-                "const int a = near_check(q, ctx, marks);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
-                "#pragma unroll", "for (int d = 0; d < kDof; d++) {", "    c[d] = q[d];",
-                '    asm volatile("" : "+f"(c[d]));', "}", f"if constexpr (Ctx::kInlineExact) return {exact}(c, ctx, marks);",
+        call = [f"if constexpr (Ctx::kInlineExact) return {exact}(c, ctx, marks);",
                 "Ctx own = ctx;   // the call must not force the caller's into memory",
                 f"const bool free = {exact}_call(c, own, marks);", "ctx.work = own.work;", "return free;"]
+        if exact != "fkcc_exact":   # single configurations: always compiled into the kernel
+            call = [f"return {exact}(c, ctx, marks);"]
+        return [f"if constexpr (Ctx::kEveryTest) return {exact}(q, ctx, AllSteps{{}});",
+                f"StepMarks<{(len(m['schedule']) + 31) // 32}> marks;   // the steps that the exact form has to make",
+                "const int a = near_check(q, ctx, marks);", "if (a != kNearUnsure) return a == kNearFree;", "float c[kDof];",
+                "#pragma unroll", "for (int d = 0; d < kDof; d++) {", "    c[d] = q[d];",
+                '    asm volatile("" : "+f"(c[d]));', "}", *call]
 
     if table:
         near_gates = near_ids
@@ -528,9 +534,12 @@ def emit_cuda_checker(m: dict) -> str:
         w("    }")
         w("};")
         w("")
-        for exact, lines in [("fkcc_exact", tcode.lines)] + ([("fkcc_validate_exact", code.lines)] if inline else []):
-            function(f"__device__ __forceinline__ bool {exact}", lines, f", const {marks_type} &marks")
-            function(f"__device__ __noinline__ bool {exact}_call", [f"return {exact}(q, ctx, marks);"], f", const {marks_type} marks")
+        w("// The exact form; marks: the steps to make (StepMarks), or AllSteps.")
+        function("__device__ __forceinline__ bool fkcc_exact", tcode.lines, ", const Marks &marks", "class Ctx, class Marks")
+        function("__device__ __noinline__ bool fkcc_exact_call", ["return fkcc_exact(q, ctx, marks);"], f", const {marks_type} marks")
+        if inline:
+            w("// The straight-line exact form makes every step, whatever the marks.")
+            function("__device__ __forceinline__ bool fkcc_validate_exact", code.lines, ", const Marks &", "class Ctx, class Marks")
         out_marks = f", {marks_type} &marks"
         function("__device__ __forceinline__ int near_check_leaves", _near_body(m, near_gates, LEAF_MARKS), out_marks)
         function("__device__ __forceinline__ int near_check_gates", _near_body(m, near_gates, ALWAYS), out_marks)
