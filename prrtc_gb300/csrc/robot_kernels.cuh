@@ -86,6 +86,13 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
     add_work(work, flops, cfgs);
 }
 
+// The checker's form for edges of more than 96 points; a robot file may specialise it.
+template <class Gen>
+struct LongEdges {
+    using Ctx = CheckCtx;
+    static constexpr int kMinBlocks = 6;
+};
+
 // Edges, a warp per 32 points of one edge: points k = 32 c + lane + 1 of edge e
 // for item c * n + e.  out holds 1 for every edge when the kernel starts; a
 // warp that meets a collision writes 0, and a warp whose edge is already known
@@ -93,8 +100,8 @@ __global__ void __launch_bounds__(ValidateLaunch<Gen>::kMaxThreads, ValidateLaun
 // edge, waiting for the block's slowest warp was a fifth of the time).
 // Chunk-major order: an edge's chunks run far apart, so that a later chunk
 // mostly finds the earlier ones' answer.
-template <class Gen>
-__global__ void __launch_bounds__(128, 6) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
+template <class Gen, class Ctx, int MinBlocks>
+__global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
                                                         const EnvGrid *grid,
                                                         const float *__restrict__ a, const float *__restrict__ b,
                                                         int64_t n, int g, uint8_t *out, unsigned long long *work)
@@ -109,7 +116,9 @@ __global__ void __launch_bounds__(128, 6) k_validate_edges(const float4 *__restr
     stage_env_bulk(s_env, env, nc.records(), &s_bar);   // synchronises the block
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     volatile int *bad = &s_bad[warp];
-    CheckCtx ctx{{s_env, nc, gr}, 0.0f, bad};
+    Ctx ctx{};
+    ctx.env = EnvView{s_env, nc, gr};
+    ctx.stop_flag = bad;
     const float fg = (float)g;
     const int64_t items = n * ((g + 31) >> 5), stride = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t it = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; it < items; it += stride) {
@@ -533,8 +542,13 @@ struct RobotKernels {
         }
         const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
         if (e != cudaSuccess) return e;
-        k_validate_edges<Gen><<<grid_for(n * chunks * 32, 128, le.sms, 16), 128, smem, st>>>(le.rec, le.counts, le.grid, a, b,
-                                                                                           n, g, out, le.work);
+        using Long = LongEdges<Gen>;
+        const int blocks = grid_for(n * chunks * 32, 128, le.sms, 16);
+        if (chunks >= 4)
+            k_validate_edges<Gen, typename Long::Ctx, Long::kMinBlocks><<<blocks, 128, smem, st>>>(
+                le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
+        else
+            k_validate_edges<Gen, CheckCtx, 6><<<blocks, 128, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
         return cudaGetLastError();
     }
     static cudaError_t fk_spheres(const float *q, int64_t n, float *out, int sms, cudaStream_t st)

@@ -83,7 +83,7 @@ def test_one_verdict_for_a_configuration(case, ctx):
     assert (out.cpu().numpy() == want).all()
 
 
-@pytest.mark.parametrize("granularity", [1, 33])
+@pytest.mark.parametrize("granularity", [1, 33, 96, 97, 128, 200])
 def test_one_verdict_for_an_edge(case, granularity, ctx):
     """Edges that stay at one point."""
     robot, _, h, plain, q, want = case
