@@ -99,7 +99,9 @@ struct LongEdges {
 // to collide skips its points.  Warps meet at no barrier (with a block per
 // edge, waiting for the block's slowest warp was a fifth of the time).
 // Chunk-major order: an edge's chunks run far apart, so that a later chunk
-// mostly finds the earlier ones' answer.
+// mostly finds the earlier ones' answer.  An edge of at most 32 points has one
+// warp, which writes its answer (no memset before the launch: 3 us of a call
+// that takes 25 to 40).
 template <class Gen, class Ctx, int MinBlocks>
 __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
                                                         const EnvGrid *grid,
@@ -124,7 +126,7 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
     for (int64_t it = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; it < items; it += stride) {
         const int64_t e = it % n;
         const int k = 32 * (int)(it / n) + lane + 1;
-        if (lane == 0) *bad = *(volatile uint8_t *)(out + e) == 0;
+        if (lane == 0) *bad = g > 32 && *(volatile uint8_t *)(out + e) == 0;
         __syncwarp();
         if (k <= g && !*bad) {
             float cfg[D];
@@ -137,12 +139,13 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
             ctx.work = 0;
             if (!Gen::fkcc(cfg, ctx)) {
                 *bad = 1;
-                out[e] = 0;
+                if (g > 32) out[e] = 0;
             }
             flops += ctx.work + Gen::kFkFlops;
             cfgs++;
         }
         __syncwarp();
+        if (g <= 32 && lane == 0) out[e] = *bad ? 0 : 1;
     }
     add_work(work, flops, cfgs);
 }
@@ -540,8 +543,10 @@ struct RobotKernels {
                 k_validate_edges_every<Gen, 0><<<blocks, threads, smem, st>>>(le.rec, le.counts, a, b, n, g, out, le.work);
             return cudaGetLastError();
         }
-        const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
-        if (e != cudaSuccess) return e;
+        if (chunks > 1) {
+            const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
+            if (e != cudaSuccess) return e;
+        }
         using Long = LongEdges<Gen>;
         const int blocks = grid_for(n * chunks * 32, 128, le.sms, 16);
         if (chunks >= 4)
