@@ -86,6 +86,13 @@ constexpr int kEarlyTrips = 4;
 constexpr float kEarlyRel = 1.0f / 1024.0f, kEarlyAbs = 1.0f / 65536.0f;
 constexpr int kEarlyBox = 8;
 
+// Warps beyond the number of queries, counted over the blocks' first warps, then
+// their second, ..., look for work this much later.  Blocks start an SM at a
+// time: without it a batch of fewer queries than warps was taken by the first
+// SMs' warps, a dozen to an SM, and the others had none (256 Fetch queries, one
+// worker each, tested against 277 obstacles 142 -> 115 ms; 16 took 100 either way).
+constexpr unsigned kLateLookNs = 4000;
+
 // warps an attempt admits: kJoinBase for its first kJoinYoungNs, then up to
 // max_workers
 constexpr int kJoinBase = 4;
@@ -593,6 +600,8 @@ __global__ void __launch_bounds__(128, 3) k_rrtc_batch(const BatchParams P)
         if (lane == 0 && nn_visits) atomicAdd(&C->nn_nodes, nn_visits);
         nn_visits = 0;
     };
+
+    if ((threadIdx.x >> 5) * gridDim.x + blockIdx.x >= (unsigned)P.num_queries) __nanosleep(kLateLookNs);
 
     while (true) {
         // ---- time budget
