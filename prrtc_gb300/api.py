@@ -455,8 +455,12 @@ class Context:
             qs["env"][is_handle] = [e.handle.value for (e, _, _), h in zip(trip, is_handle) if h]
         plain = np.flatnonzero(~is_handle)
         if len(plain):
-            descs = np.zeros(len(plain), _DESC_DT)
-            envs = [trip[i][0] for i in plain]
+            # one descriptor per distinct environment object: queries that share
+            # it share its records and clearance grid in the library
+            number = {}
+            which = np.fromiter((number.setdefault(id(trip[i][0]), len(number)) for i in plain), np.int64, len(plain))
+            envs = [trip[i][0] for i in plain[np.unique(which, return_index=True)[1]]]
+            descs = np.zeros(len(envs), _DESC_DT)
             packed = all(type(e) is Environment for e in envs)   # float32, contiguous, [count, width] already
             for k in _ENV_KINDS:                       # one buffer per obstacle type, descriptors point into it
                 arrs = [getattr(e, k) for e in envs] if packed else \
@@ -469,7 +473,7 @@ class Context:
                     descs[k] = np.where(cnt > 0, ptr, 0)
                 descs["num_" + k] = cnt
             keep.append(descs)
-            qs["env_desc"][plain] = descs.ctypes.data + _DESC_DT.itemsize * np.arange(len(plain), dtype=np.uint64)
+            qs["env_desc"][plain] = descs.ctypes.data + _DESC_DT.itemsize * which.astype(np.uint64)
         paths = np.empty((n, path_capacity, D), np.float32)
         res = np.zeros(n, _RESULT_DT)
         res["path_capacity"] = path_capacity
@@ -539,6 +543,7 @@ class Batch:
         self.n = len(queries)
         self.path_capacity = path_capacity
         self._keep = []
+        descs = {}   # one per distinct environment object
         qs = (_Query * self.n)()
         for i, q in enumerate(queries):
             env, start, goals = q if isinstance(q, tuple) else (q.env, q.start, q.goal)
@@ -548,9 +553,11 @@ class Batch:
             if isinstance(env, EnvHandle):
                 qs[i].env = env.handle
             else:
-                d, keep = _env_desc(env)
-                self._keep += [d, keep]
-                qs[i].env_desc = C.cast(C.pointer(d), C.c_void_p)
+                if id(env) not in descs:
+                    d, keep = _env_desc(env)
+                    self._keep += [env, d, keep]
+                    descs[id(env)] = C.cast(C.pointer(d), C.c_void_p)
+                qs[i].env_desc = descs[id(env)]
             qs[i].start = start.ctypes.data
             qs[i].goals = goals.ctypes.data
             qs[i].num_goals = len(goals)

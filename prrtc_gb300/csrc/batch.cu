@@ -26,6 +26,20 @@ struct Arena {
     bool in_use = false;
 };
 
+// Device memory; the idle memory kept for grids is given up for it if need be.
+static cudaError_t alloc(Ctx *c, void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess && !c->grids_in_use && c->grids.ptr) {
+        cudaGetLastError();
+        cudaFree(c->grids.ptr);
+        c->grids = {};
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
 static void arena_free(Arena *a)
 {
     if (!a) return;
@@ -44,9 +58,10 @@ void release_arena(Ctx *c)
 }
 
 // Memory for a batch's clearance grids: the context's, kept between batches
-// (allocating and freeing 135 MB took 0.25 ms of a 1024-query call), or the
-// batch's own while another batch holds that one.  Null: no room.
-static constexpr size_t kGridsKept = (size_t)1 << 30;
+// (allocating and freeing 135 MB took 0.25 ms of a 1024-query call, 2.8 GB
+// several of a call with 20 480 scenes), or the batch's own while another batch
+// holds that one.  Null: no room.
+static constexpr size_t kGridsKept = (size_t)4 << 30;
 
 static char *take_grids(Ctx *c, size_t bytes)
 {
@@ -97,9 +112,9 @@ static prrtc_status take_arena(Ctx *c, int dof, int cap, int slots, Arena **out)
     a->cap = cap;
     a->slots = slots;
     const size_t nn = (size_t)slots * 2 * dof * cap, np = (size_t)slots * 2 * cap;
-    if (cudaMalloc(&a->nodes, nn * sizeof(float)) != cudaSuccess || cudaMalloc(&a->parents, np * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&a->radii, np * sizeof(float)) != cudaSuccess) {
-        cudaGetLastError();
+    if (alloc(c, (void **)&a->nodes, nn * sizeof(float)) != cudaSuccess ||
+        alloc(c, (void **)&a->parents, np * sizeof(int)) != cudaSuccess ||
+        alloc(c, (void **)&a->radii, np * sizeof(float)) != cudaSuccess) {
         arena_free(a);
         return c->fail(PRRTC_ENOMEM, "batch: cannot allocate an arena of %d slots x %d nodes", slots, cap);
     }
@@ -154,10 +169,50 @@ struct prrtc_batch {
     bool ran = false;
 };
 
-// cells of a query's own clearance grid (135 KB; 8-10 cm cells on the
+// cells of a host scene's clearance grid (135 KB; 8-10 cm cells on the
 // tabletop and shelf scenes), and the most memory a batch spends on them
 static constexpr int kBatchCells = 4096;
 static constexpr size_t kGridBytes = (size_t)8 << 30;
+
+// Queries that bring the same obstacle arrays share one scene: its records are
+// packed and uploaded and its grid is built once.  The arrays are compared by
+// address and count, which is enough within one call.
+class SceneTable {
+  public:
+    explicit SceneTable(int n)
+    {
+        size_t slots = 16;
+        while (slots < 2 * (size_t)n) slots *= 2;
+        first_.assign(slots, -1);
+        keys_.resize(n);
+    }
+    // the first query that came with e's arrays: i itself if none did before
+    int add(int i, const prrtc_env_desc &e)
+    {
+        const float *p[5] = {e.spheres, e.capsules, e.z_aligned_capsules, e.cuboids, e.z_aligned_cuboids};
+        const uint32_t n[5] = {e.num_spheres, e.num_capsules, e.num_z_aligned_capsules, e.num_cuboids, e.num_z_aligned_cuboids};
+        uint64_t h = 0;
+        for (int k = 0; k < 5; k++) {
+            keys_[i].p[k] = n[k] ? p[k] : nullptr;
+            keys_[i].n[k] = n[k];
+            h = (h ^ (uint64_t)(uintptr_t)keys_[i].p[k] ^ ((uint64_t)n[k] << 48)) * 0x9E3779B97F4A7C15ull;
+            h ^= h >> 29;
+        }
+        for (size_t s = h & (first_.size() - 1);; s = (s + 1) & (first_.size() - 1)) {
+            if (first_[s] < 0) return first_[s] = i;
+            const Key &o = keys_[first_[s]];
+            if (std::equal(o.p, o.p + 5, keys_[i].p) && std::equal(o.n, o.n + 5, keys_[i].n)) return first_[s];
+        }
+    }
+
+  private:
+    struct Key {
+        const float *p[5];
+        uint32_t n[5];
+    };
+    std::vector<Key> keys_;
+    std::vector<int> first_;
+};
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -190,6 +245,8 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
     // configurations and obstacle records are allocated once and written in
     // place, with no per-query temporaries
     size_t cfg_floats = 0, env_records = 0;
+    std::vector<int> scene(n, -1);   // the first query with the same host obstacles
+    SceneTable scenes(n);
     for (int i = 0; i < n; i++) {
         const prrtc_query &q = queries[i];
         if (!q.start || !q.goals || q.num_goals < 1 || q.num_goals >= cap || (!q.env && !q.env_desc))
@@ -200,14 +257,15 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
             const uint64_t recs = (uint64_t)e.num_spheres + 2ull * e.num_capsules + 2ull * e.num_z_aligned_capsules +
                                   4ull * e.num_cuboids + 4ull * e.num_z_aligned_cuboids;
             if (recs * 4 > (uint64_t)PRRTC_MAX_ENV_FLOATS) return c->fail(PRRTC_EINVAL, "batch_create: env %d too large", i);
-            env_records += recs;
+            scene[i] = scenes.add(i, e);
+            if (scene[i] == i) env_records += recs;
         }
     }
     std::vector<float> cfg;
     std::vector<float4> envs;
     cfg.reserve(cfg_floats);
     envs.reserve(env_records);
-    std::vector<BatchQueryDesc> descs(n);
+    std::vector<BatchQueryDesc> descs(n, BatchQueryDesc{});
     std::vector<int> env_rec_off(n, -1);
     for (int i = 0; i < n; i++) {
         const prrtc_query &q = queries[i];
@@ -220,7 +278,8 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
             descs[i].env = e->dev;
             descs[i].env_n = e->counts;
             descs[i].grid = e->grid;
-            descs[i].build = 0;
+        } else if (scene[i] != i) {
+            descs[i].env_n = descs[scene[i]].env_n;
         } else {
             const prrtc_env_desc &e = *q.env_desc;
             env_rec_off[i] = (int)envs.size();
@@ -256,6 +315,8 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
     off = align256(off + std::max<size_t>(1, envs.size()) * sizeof(float4));
     const size_t o_desc = off;
     off = align256(off + n * sizeof(BatchQueryDesc));
+    const size_t o_scenes = off;   // the scenes whose grids are built
+    off = align256(off + (std::count_if(scene.begin(), scene.end(), [](int v) { return v >= 0; })) * sizeof(BatchQueryDesc));
     const size_t o_order = off;
     off = align256(off + n * sizeof(int));
     const size_t o_qstate = off;
@@ -269,33 +330,48 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
     const size_t o_path = off;
     off = align256(off + (size_t)b->path_rows * D * sizeof(float));
     prrtc_status s;
-    if (cudaMalloc(&b->blob, off) != cudaSuccess) {
-        cudaGetLastError();
+    if (alloc(c, &b->blob, off) != cudaSuccess) {
         delete b;
         return c->fail(PRRTC_ENOMEM, "batch_create: cannot allocate %zu bytes", off);
     }
-    // queries that bring host obstacles get a clearance grid of their own, if
-    // there is room for them (without it the checker tests every obstacle)
-    size_t own_envs = 0, own = 0;
-    for (int i = 0; i < n; i++) own_envs += env_rec_off[i] >= 0 && descs[i].env_n.obstacles() > 0;
+    if ((s = take_arena(c, D, cap, slots, &b->arena))) {
+        prrtc_batch_free(ctx, b);
+        return s;
+    }
+    // host scenes get a clearance grid each, if there is room left for them
+    // (without it the checker tests every obstacle)
+    std::vector<BatchQueryDesc> own;   // the scenes whose grids are built
+    auto can_have_grid = [&](int i) {
+        return scene[i] == i && descs[i].env_n.obstacles() >= 1 && descs[i].env_n.obstacles() <= kGridMaxObstacles;
+    };
+    size_t grids = 0;
+    for (int i = 0; i < n; i++) grids += can_have_grid(i);
     const size_t grid_bytes = env_grid_bytes(kBatchCells);
-    if (own_envs > 0 && own_envs * grid_bytes <= kGridBytes) b->grids = take_grids(c, own_envs * grid_bytes);
+    if (grids > 0 && grids * grid_bytes <= kGridBytes) b->grids = take_grids(c, grids * grid_bytes);
     char *base = static_cast<char *>(b->blob);
     float4 *env_dev = reinterpret_cast<float4 *>(base + o_env);
-    for (int i = 0; i < n; i++)
-        if (env_rec_off[i] >= 0) {
-            descs[i].env = env_dev + env_rec_off[i];
-            const bool grid = b->grids && descs[i].env_n.obstacles() > 0;
-            descs[i].grid = grid ? reinterpret_cast<const EnvGrid *>(b->grids + grid_bytes * own++) : nullptr;
-            descs[i].build = grid;
+    for (int i = 0; i < n; i++) {
+        if (scene[i] < 0) continue;
+        BatchQueryDesc &d = descs[i];
+        if (scene[i] == i) {
+            d.env = env_dev + env_rec_off[i];
+            if (b->grids && can_have_grid(i)) {
+                d.grid = reinterpret_cast<const EnvGrid *>(b->grids + grid_bytes * own.size());
+                own.push_back(d);
+            }
+        } else {
+            d.env = descs[scene[i]].env;
+            d.grid = descs[scene[i]].grid;
         }
+    }
     if ((s = ensure_halton_bases(c, b->lanes * max_attempts)) ||
         (s = c->cuda(cudaMemcpyAsync(base + o_cfg, cfg.data(), cfg.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream), "batch upload")) ||
         (!envs.empty() && (s = c->cuda(cudaMemcpyAsync(env_dev, envs.data(), envs.size() * sizeof(float4), cudaMemcpyHostToDevice, c->stream), "batch upload"))) ||
         (s = c->cuda(cudaMemcpyAsync(base + o_desc, descs.data(), n * sizeof(BatchQueryDesc), cudaMemcpyHostToDevice, c->stream), "batch upload")) ||
-        (own && (s = c->cuda(launch_env_grids(reinterpret_cast<const BatchQueryDesc *>(base + o_desc), n, BatchQueryDesc{},
-                                              kBatchCells, c->stream), "batch grids"))) ||
-        (s = take_arena(c, D, cap, slots, &b->arena)) ||
+        (!own.empty() &&
+         ((s = c->cuda(cudaMemcpyAsync(base + o_scenes, own.data(), own.size() * sizeof(BatchQueryDesc), cudaMemcpyHostToDevice, c->stream), "batch upload")) ||
+          (s = c->cuda(launch_env_grids(reinterpret_cast<const BatchQueryDesc *>(base + o_scenes), (int)own.size(), kBatchCells,
+                                        c->stream), "batch grids")))) ||
         (s = c->cuda(cudaEventCreate(&b->ev0), "event")) || (s = c->cuda(cudaEventCreate(&b->ev1), "event")) ||
         (s = c->cuda(cudaStreamSynchronize(c->stream), "batch upload"))) {
         prrtc_batch_free(ctx, b);

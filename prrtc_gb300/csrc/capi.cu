@@ -293,7 +293,8 @@ prrtc_status prrtc_env_upload(prrtc_ctx *ctx, const prrtc_env_desc *d, prrtc_env
         const size_t rec_bytes = e->host.size() * sizeof(float4);
         // room for the grid if these obstacles can have one and there is any
         // (without it the checker tests every obstacle)
-        bool grid = env_grid_usable(e->host.data(), e->counts);
+        EnvGrid header;
+        bool grid = env_grid_header(e->host.data(), e->counts, kEnvCells, &header);
         if (grid && cudaMalloc(&e->dev, rec_bytes + env_grid_bytes(kEnvCells)) != cudaSuccess) {
             cudaGetLastError();
             grid = false;
@@ -303,14 +304,10 @@ prrtc_status prrtc_env_upload(prrtc_ctx *ctx, const prrtc_env_desc *d, prrtc_env
             delete e;
             return c->fail(PRRTC_ENOMEM, "env_upload: cudaMalloc failed");
         }
-        BatchQueryDesc d{};
-        d.env = e->dev;
-        d.env_n = e->counts;
-        d.grid = e->grid = grid ? reinterpret_cast<const EnvGrid *>(e->dev + e->host.size()) : nullptr;
-        d.build = 1;
+        if (grid) e->grid = reinterpret_cast<const EnvGrid *>(e->dev + e->host.size());
         prrtc_status s;
         if ((s = c->cuda(cudaMemcpyAsync(e->dev, e->host.data(), rec_bytes, cudaMemcpyHostToDevice, c->stream), "env_upload copy")) ||
-            (grid && (s = c->cuda(launch_env_grids(nullptr, 1, d, kEnvCells, c->stream), "env_upload grid"))) ||
+            (grid && (s = c->cuda(launch_env_grid(header, e->dev, e->grid, kEnvCells, c->stream), "env_upload grid"))) ||
             (s = c->cuda(cudaStreamSynchronize(c->stream), "env_upload"))) {
             cudaFree(e->dev);
             delete e;

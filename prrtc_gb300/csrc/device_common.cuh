@@ -263,7 +263,7 @@ __device__ __forceinline__ int env_cost(const EnvCounts &n, int k)
     return a * kFlopSphere + b * kFlopCapsule + c * kFlopZCapsule + d * kFlopCuboid + (k - d) * kFlopZCuboid;
 }
 
-__device__ __forceinline__ int env_cost_all(const EnvCounts &n)
+__host__ __device__ __forceinline__ int env_cost_all(const EnvCounts &n)
 {
     return n.ns * kFlopSphere + n.nc * kFlopCapsule + n.nzc * kFlopZCapsule + n.ncb * kFlopCuboid + n.nzb * kFlopZCuboid;
 }

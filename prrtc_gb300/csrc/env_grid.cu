@@ -113,80 +113,98 @@ __device__ __forceinline__ void insert(unsigned (&key)[16], unsigned v)
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__restrict__ many, BatchQueryDesc one,
-                                                      int max_cells)
+// The header of a grid over the box b around usable obstacles (ok), and where
+// it and what it points to lie.
+__host__ __device__ void place(EnvGrid &g, const float4 *rec, const EnvGrid *where, int max_cells)
 {
-    const BatchQueryDesc Q = many ? many[blockIdx.y] : one;
-    if (!Q.build) return;
-    const float4 *rec = Q.env;
-    const EnvCounts n = Q.env_n;
-    const int no = n.obstacles();
+    g.rec = rec;
+    g.near_ = reinterpret_cast<const uint8_t *>(where + 1);
+    g.list = reinterpret_cast<const uint4 *>(g.near_ + max_cells);
+}
+
+__host__ __device__ EnvGrid make_header(const Box &b, bool ok, const EnvCounts &n, int max_cells)
+{
+    EnvGrid g{};
+    g.out_r = -1.0f;
+    float cells[3], from[3], ext[3];
+    for (int i = 0; i < 3; i++) {
+        g.lo[i] = ok ? b.lo[i] : 1.0f;
+        g.hi[i] = ok ? b.hi[i] : -1.0f;
+        from[i] = fmaxf(b.lo[i] - kInflate, -kRoom);
+        ext[i] = fminf(b.hi[i] + kInflate, kRoom) - from[i];
+    }
+    g.cost = env_cost_all(n);
+    g.counts = n;
+    if (ok && ext[0] > 1e-3f && ext[1] > 1e-3f && ext[2] > 1e-3f) {
+        // cubic cells, at most max_cells of them
+        const float size = cbrtf(ext[0] * ext[1] * ext[2] / (float)max_cells);
+        for (int i = 0; i < 3; i++) cells[i] = fmaxf(1.0f, fminf(128.0f, floorf(ext[i] / size)));
+        g.out_r = 0.95f * kInflate;
+        while (cells[0] * cells[1] * cells[2] > (float)max_cells) {
+            const int i = cells[0] >= cells[1] && cells[0] >= cells[2] ? 0 : cells[1] >= cells[2] ? 1 : 2;
+            cells[i] -= 1.0f;
+        }
+        for (int i = 0; i < 3; i++) {
+            g.n[i] = (int)cells[i];
+            g.inv[i] = cells[i] / ext[i];
+            g.off[i] = -from[i] * g.inv[i] - 0.5f;
+            if (b.lo[i] - kInflate < -kRoom || b.hi[i] + kInflate > kRoom) g.out_r = -1.0f;
+        }
+    }
+    return g;
+}
+
+// Scene blockIdx.y of `scenes`, its header from its records; without `scenes`
+// the one grid of header `one`.
+__global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__restrict__ scenes, EnvGrid one, int max_cells)
+{
     __shared__ Box s_box[kThreads / 32];
     __shared__ EnvGrid s_g;
-    // the box around the obstacles (every block for itself: at most 255 obstacles)
-    Box b;
-    for (int i = 0; i < 3; i++) {
-        b.lo[i] = 1e30f;
-        b.hi[i] = -1e30f;
-    }
-    bool ok = no >= 1 && no <= kGridMaxObstacles;
-    if (ok)
-        for (int k = threadIdx.x; k < no; k += kThreads) {
-            Box o;
-            ok = obstacle_box(rec, n, k, o) && ok;
-            for (int i = 0; i < 3; i++) {
-                b.lo[i] = fminf(b.lo[i], o.lo[i]);
-                b.hi[i] = fmaxf(b.hi[i], o.hi[i]);
-            }
-        }
-    for (int i = 0; i < 3; i++)
-        for (int off = 16; off > 0; off >>= 1) {
-            b.lo[i] = fminf(b.lo[i], __shfl_xor_sync(0xffffffffu, b.lo[i], off));
-            b.hi[i] = fmaxf(b.hi[i], __shfl_xor_sync(0xffffffffu, b.hi[i], off));
-        }
-    if ((threadIdx.x & 31) == 0) s_box[threadIdx.x >> 5] = b;
-    ok = __syncthreads_and(ok);
-    if (threadIdx.x == 0) {
-        EnvGrid g{};
-        g.out_r = -1.0f;
-        float cells[3], from[3], ext[3];
+    if (!scenes) {
+        if (threadIdx.x == 0) s_g = one;
+    } else {
+        const BatchQueryDesc Q = scenes[blockIdx.y];
+        // the box around the obstacles (every block for itself: at most 255 obstacles)
+        Box b;
         for (int i = 0; i < 3; i++) {
-            for (int w = 1; w < kThreads / 32; w++) {
-                b.lo[i] = fminf(b.lo[i], s_box[w].lo[i]);
-                b.hi[i] = fmaxf(b.hi[i], s_box[w].hi[i]);
-            }
-            g.lo[i] = ok ? b.lo[i] : 1.0f;
-            g.hi[i] = ok ? b.hi[i] : -1.0f;
-            from[i] = fmaxf(b.lo[i] - kInflate, -kRoom);
-            ext[i] = fminf(b.hi[i] + kInflate, kRoom) - from[i];
+            b.lo[i] = 1e30f;
+            b.hi[i] = -1e30f;
         }
-        g.near_ = reinterpret_cast<const uint8_t *>(Q.grid + 1);
-        g.list = reinterpret_cast<const uint4 *>(g.near_ + max_cells);
-        g.cost = env_cost(n, no);
-        g.counts = n;
-        g.rec = rec;
-        if (ok && ext[0] > 1e-3f && ext[1] > 1e-3f && ext[2] > 1e-3f) {
-            // cubic cells, at most max_cells of them
-            const float size = cbrtf(ext[0] * ext[1] * ext[2] / (float)max_cells);
-            for (int i = 0; i < 3; i++) cells[i] = fmaxf(1.0f, fminf(128.0f, floorf(ext[i] / size)));
-            g.out_r = 0.95f * kInflate;
-            while (cells[0] * cells[1] * cells[2] > (float)max_cells) {
-                const int i = cells[0] >= cells[1] && cells[0] >= cells[2] ? 0 : cells[1] >= cells[2] ? 1 : 2;
-                cells[i] -= 1.0f;
+        const int no = Q.env_n.obstacles();
+        bool ok = no >= 1 && no <= kGridMaxObstacles;
+        if (ok)
+            for (int k = threadIdx.x; k < no; k += kThreads) {
+                Box o;
+                ok = obstacle_box(Q.env, Q.env_n, k, o) && ok;
+                for (int i = 0; i < 3; i++) {
+                    b.lo[i] = fminf(b.lo[i], o.lo[i]);
+                    b.hi[i] = fmaxf(b.hi[i], o.hi[i]);
+                }
             }
-            for (int i = 0; i < 3; i++) {
-                g.n[i] = (int)cells[i];
-                g.inv[i] = cells[i] / ext[i];
-                g.off[i] = -from[i] * g.inv[i] - 0.5f;
-                if (b.lo[i] - kInflate < -kRoom || b.hi[i] + kInflate > kRoom) g.out_r = -1.0f;
+        for (int i = 0; i < 3; i++)
+            for (int off = 16; off > 0; off >>= 1) {
+                b.lo[i] = fminf(b.lo[i], __shfl_xor_sync(0xffffffffu, b.lo[i], off));
+                b.hi[i] = fmaxf(b.hi[i], __shfl_xor_sync(0xffffffffu, b.hi[i], off));
             }
+        if ((threadIdx.x & 31) == 0) s_box[threadIdx.x >> 5] = b;
+        ok = __syncthreads_and(ok);
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kThreads / 32; w++)
+                for (int i = 0; i < 3; i++) {
+                    b.lo[i] = fminf(b.lo[i], s_box[w].lo[i]);
+                    b.hi[i] = fmaxf(b.hi[i], s_box[w].hi[i]);
+                }
+            s_g = make_header(b, ok, Q.env_n, max_cells);
+            place(s_g, Q.env, Q.grid, max_cells);
         }
-        s_g = g;
-        if (blockIdx.x == 0) *const_cast<EnvGrid *>(Q.grid) = g;
     }
+    if (threadIdx.x == 0 && blockIdx.x == 0)   // the header lies in front of the bounds
+        *(reinterpret_cast<EnvGrid *>(const_cast<uint8_t *>(s_g.near_)) - 1) = s_g;
     __syncthreads();
     const int cell = blockIdx.x * kThreads + threadIdx.x;
     if (cell >= s_g.n[0] * s_g.n[1] * s_g.n[2]) return;
+    const float4 *rec = s_g.rec;
+    const EnvCounts n = s_g.counts;
     // the cell: centre and half-extents, a little larger than the cut (a
     // point's cell is rounded)
     const int ix = cell % s_g.n[0], iy = cell / s_g.n[0] % s_g.n[1], iz = cell / (s_g.n[0] * s_g.n[1]);
@@ -264,21 +282,36 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
 
 // (the lists, 16-byte entries, follow the header and a multiple of 16 bytes)
 static_assert(sizeof(EnvGrid) % 16 == 0, "the lists behind the header are 16-byte entries");
-bool env_grid_usable(const float4 *rec, const EnvCounts &n)
+bool env_grid_header(const float4 *host_rec, const EnvCounts &n, int cells, EnvGrid *out)
 {
-    Box b;
-    bool ok = n.obstacles() >= 1 && n.obstacles() <= kGridMaxObstacles;
-    for (int k = 0; ok && k < n.obstacles(); k++) ok = obstacle_box(rec, n, k, b);
-    return ok;
+    Box all{{1e30f, 1e30f, 1e30f}, {-1e30f, -1e30f, -1e30f}};
+    if (n.obstacles() < 1 || n.obstacles() > kGridMaxObstacles) return false;
+    for (int k = 0; k < n.obstacles(); k++) {
+        Box b;
+        if (!obstacle_box(host_rec, n, k, b)) return false;
+        for (int i = 0; i < 3; i++) {
+            all.lo[i] = std::min(all.lo[i], b.lo[i]);
+            all.hi[i] = std::max(all.hi[i], b.hi[i]);
+        }
+    }
+    *out = make_header(all, true, n, cells);
+    return true;
 }
 
 size_t env_grid_bytes(int cells) { return sizeof(EnvGrid) + (size_t)cells * 33; }
 
-cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st)
+cudaError_t launch_env_grid(EnvGrid header, const float4 *rec, const EnvGrid *where, int cells, cudaStream_t st)
+{
+    place(header, rec, where, cells);
+    k_env_grid<<<(cells + kThreads - 1) / kThreads, kThreads, 0, st>>>(nullptr, header, cells);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_env_grids(const BatchQueryDesc *scenes, int n, int cells, cudaStream_t st)
 {
     for (int first = 0; first < n; first += 65535) {
         const dim3 grid((cells + kThreads - 1) / kThreads, std::min(n - first, 65535));
-        k_env_grid<<<grid, kThreads, 0, st>>>(many ? many + first : nullptr, one, cells);
+        k_env_grid<<<grid, kThreads, 0, st>>>(scenes + first, EnvGrid{}, cells);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -67,7 +67,6 @@ struct BatchQueryDesc {
     int cfg_off;         // float offset of start (dof floats) then goals in the config pool
     int num_goals;
     const EnvGrid *grid; // clearance grid (device), or none
-    int build;           // 1: the batch builds the grid (an uploaded environment brings its own)
 };
 
 enum SlotStateCode { SLOT_FREE = 0, SLOT_RUNNING = 1, SLOT_DONE = 2, SLOT_BUSY = 3 };
@@ -206,11 +205,14 @@ struct GoalQuery {
 };
 
 // Clearance grids (env_grid.cu): device bytes of one with at most `cells`
-// cells (a multiple of 16), and the launch that builds those of the n
-// descriptors that ask for it (device array `many`, or the single `one`).
+// cells (a multiple of 16); the header of one from the host's copy of the
+// records (false: these obstacles cannot have a grid) and the launch that
+// builds it at `where`; and the launch that builds those of n scenes (device
+// array; a scene that cannot have one gets a header that says so).
 size_t env_grid_bytes(int cells);
-bool env_grid_usable(const float4 *rec, const EnvCounts &n);   // (host records) may there be a grid?
-cudaError_t launch_env_grids(const BatchQueryDesc *many, int n, const BatchQueryDesc &one, int cells, cudaStream_t st);
+bool env_grid_header(const float4 *host_rec, const EnvCounts &n, int cells, EnvGrid *out);
+cudaError_t launch_env_grid(EnvGrid header, const float4 *rec, const EnvGrid *where, int cells, cudaStream_t st);
+cudaError_t launch_env_grids(const BatchQueryDesc *scenes, int n, int cells, cudaStream_t st);
 
 struct ClrLaunch;   // clearance_device.cuh
 struct ClrModel;

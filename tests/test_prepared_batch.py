@@ -41,3 +41,21 @@ def test_prepared_arrays_point_at_the_host_data():
                 assert not getattr(d, k), (i, k)
         r = prep.res[i]
         assert r["path_capacity"] == 16 and int(r["path"]) == prep.paths[i].ctypes.data
+
+
+def test_queries_of_one_environment_share_its_descriptor():
+    from prrtc_gb300 import Context, Environment
+    from prrtc_gb300.api import EnvDesc
+    rng = np.random.default_rng(1)
+    a, b = Environment(spheres=rng.random((3, 4))), Environment(spheres=rng.random((2, 4)))
+    q = rng.random(7).astype(np.float32)
+    ctx = Context.__new__(Context)
+    ctx.handle = None
+    order = [b, a, a, b, Environment(spheres=a.spheres.copy()), a]
+    prep = ctx.prepare_batch("panda", [(e, q, q) for e in order], path_capacity=4)
+    at = prep.qs["env_desc"].tolist()
+    assert at[0] == at[3] and at[1] == at[2] == at[5] and len(set(at)) == 3
+    for e, addr in zip(order, at):
+        d = EnvDesc.from_address(int(addr))
+        assert d.num_spheres == len(e.spheres)
+        np.testing.assert_array_equal(floats_at(d.spheres, e.spheres.size).reshape(-1, 4), e.spheres)
