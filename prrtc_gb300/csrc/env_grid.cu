@@ -4,8 +4,9 @@
 //
 // One thread per cell walks the obstacles in their order, bounds the distance
 // from the cell to each from below, and keeps the 16 nearest by a chain of
-// min / max in registers.  What bounds the build is that arithmetic: ~60
-// instructions per obstacle and cell, the records read as broadcasts.
+// min / max in registers.  What bounds the build of many is that arithmetic, ~60
+// instructions per obstacle and cell; of one, its latency, so the records come
+// to shared memory first and an upload's header is made on the host.
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -154,12 +155,89 @@ __host__ __device__ EnvGrid make_header(const Box &b, bool ok, const EnvCounts &
     return g;
 }
 
+// Bounds and list of one cell; rec: the obstacles in shared memory.
+__device__ __forceinline__ void build_cell(const EnvGrid &g, const float4 *rec, const EnvCounts &n, int cell)
+{
+    // the cell: centre and half-extents, a little larger than the cut (a
+    // point's cell is rounded)
+    const int ix = cell % g.n[0], iy = cell / g.n[0] % g.n[1], iz = cell / (g.n[0] * g.n[1]);
+    const float cx = ((float)ix - g.off[0]) / g.inv[0], cy = ((float)iy - g.off[1]) / g.inv[1],
+                cz = ((float)iz - g.off[2]) / g.inv[2];
+    const float hx = 0.5005f / g.inv[0], hy = 0.5005f / g.inv[1], hz = 0.5005f / g.inv[2];
+    const float hd = sqrtf(hx * hx + hy * hy + hz * hz);
+    unsigned key[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) key[i] = 0xFFFFu;
+    const float4 *p = rec;
+    int k = 0;
+    for (int i = 0; i < n.ns; i++, k++) {
+        const float4 s = p[i];
+        insert(key, bound_key(gap(cx - s.x, cy - s.y, cz - s.z, hx, hy, hz) - fabsf(s.w), k));
+    }
+    p += n.ns;
+    for (int i = 0; i < n.nc + n.nzc; i++, k++) {
+        const float4 a = p[2 * i];
+        float4 v = p[2 * i + 1];
+        if (i >= n.nc) v.x = v.y = 0.0f;
+        const float dx = cx - a.x, dy = cy - a.y, dz = cz - a.z, vv = v.x * v.x + v.y * v.y + v.z * v.z;
+        const float t = vv > 0.0f ? clamp01((dx * v.x + dy * v.y + dz * v.z) / vv) : 0.0f;
+        const float ex = dx - t * v.x, ey = dy - t * v.y, ez = dz - t * v.z;
+        insert(key, bound_key(sqrtf(ex * ex + ey * ey + ez * ez) - hd - fabsf(a.w), k));
+    }
+    p += 2 * (n.nc + n.nzc);
+    for (int i = 0; i < n.ncb + n.nzb; i++, k++) {
+        const float4 c0 = p[4 * i], c1 = p[4 * i + 1], c2 = p[4 * i + 2], c3 = p[4 * i + 3];
+        const float dx = cx - c0.x, dy = cy - c0.y, dz = cz - c0.z;
+        auto term = [&](float ax, float ay, float az, float h) {
+            return fmaxf(fabsf(ax * dx + ay * dy + az * dz) - h - (fabsf(ax) * hx + fabsf(ay) * hy + fabsf(az) * hz), 0.0f);
+        };
+        const bool up = i >= n.ncb;
+        const float t1 = term(c1.x, c1.y, up ? 0.0f : c1.z, c0.w), t2 = term(c2.x, c2.y, up ? 0.0f : c2.z, c1.w),
+                    t3 = up ? term(0.0f, 0.0f, 1.0f, c2.w) : term(c3.x, c3.y, c3.z, c2.w);
+        insert(key, bound_key(sqrtf(t1 * t1 + t2 * t2 + t3 * t3), k));
+    }
+    const unsigned next = key[15] >> 8;
+    const_cast<uint8_t *>(g.near_)[cell] = (uint8_t)(key[0] >> 8);
+    // the listed ones by obstacle number (a bitonic network; unused entries last)
+    key[15] = 0xFFFFu;
+#pragma unroll
+    for (int i = 0; i < 16; i++) key[i] = ((key[i] & 255u) << 8) | (key[i] >> 8);
+#pragma unroll
+    for (int size = 2; size <= 16; size <<= 1)
+#pragma unroll
+        for (int step = size >> 1; step > 0; step >>= 1)
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const int j = i ^ step;
+                if (j > i) {
+                    const unsigned lo = min(key[i], key[j]), hi = max(key[i], key[j]);
+                    key[i] = (i & size) ? hi : lo;
+                    key[j] = (i & size) ? lo : hi;
+                }
+            }
+    unsigned lb[4], num[4];
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        lb[w] = num[w] = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const unsigned v = 4 * w + i == 15 ? 0xFF00u | next : key[4 * w + i];
+            lb[w] |= (v & 255u) << (8 * i);
+            num[w] |= (v >> 8) << (8 * i);
+        }
+    }
+    uint4 *L = const_cast<uint4 *>(g.list) + 2 * (size_t)cell;
+    L[0] = make_uint4(lb[0], lb[1], lb[2], lb[3]);
+    L[1] = make_uint4(num[0], num[1], num[2], num[3]);
+}
+
 // Scene blockIdx.y of `scenes`, its header from its records; without `scenes`
 // the one grid of header `one`.
 __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__restrict__ scenes, EnvGrid one, int max_cells)
 {
     __shared__ Box s_box[kThreads / 32];
     __shared__ EnvGrid s_g;
+    __shared__ float4 s_rec[4 * kGridMaxObstacles];
     if (!scenes) {
         if (threadIdx.x == 0) s_g = one;
     } else {
@@ -201,83 +279,13 @@ __global__ void __launch_bounds__(kThreads) k_env_grid(const BatchQueryDesc *__r
     if (threadIdx.x == 0 && blockIdx.x == 0)   // the header lies in front of the bounds
         *(reinterpret_cast<EnvGrid *>(const_cast<uint8_t *>(s_g.near_)) - 1) = s_g;
     __syncthreads();
-    const int cell = blockIdx.x * kThreads + threadIdx.x;
-    if (cell >= s_g.n[0] * s_g.n[1] * s_g.n[2]) return;
-    const float4 *rec = s_g.rec;
+    const int cells = s_g.n[0] * s_g.n[1] * s_g.n[2];
+    if (cells == 0) return;
     const EnvCounts n = s_g.counts;
-    // the cell: centre and half-extents, a little larger than the cut (a
-    // point's cell is rounded)
-    const int ix = cell % s_g.n[0], iy = cell / s_g.n[0] % s_g.n[1], iz = cell / (s_g.n[0] * s_g.n[1]);
-    const float cx = ((float)ix - s_g.off[0]) / s_g.inv[0], cy = ((float)iy - s_g.off[1]) / s_g.inv[1],
-                cz = ((float)iz - s_g.off[2]) / s_g.inv[2];
-    const float hx = 0.5005f / s_g.inv[0], hy = 0.5005f / s_g.inv[1], hz = 0.5005f / s_g.inv[2];
-    const float hd = sqrtf(hx * hx + hy * hy + hz * hz);
-    unsigned key[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) key[i] = 0xFFFFu;
-    const float4 *p = rec;
-    int k = 0;
-    for (int i = 0; i < n.ns; i++, k++) {
-        const float4 s = __ldg(p + i);
-        insert(key, bound_key(gap(cx - s.x, cy - s.y, cz - s.z, hx, hy, hz) - fabsf(s.w), k));
-    }
-    p += n.ns;
-    for (int i = 0; i < n.nc + n.nzc; i++, k++) {
-        const float4 a = __ldg(p + 2 * i);
-        float4 v = __ldg(p + 2 * i + 1);
-        if (i >= n.nc) v.x = v.y = 0.0f;
-        const float dx = cx - a.x, dy = cy - a.y, dz = cz - a.z, vv = v.x * v.x + v.y * v.y + v.z * v.z;
-        const float t = vv > 0.0f ? clamp01((dx * v.x + dy * v.y + dz * v.z) / vv) : 0.0f;
-        const float ex = dx - t * v.x, ey = dy - t * v.y, ez = dz - t * v.z;
-        insert(key, bound_key(sqrtf(ex * ex + ey * ey + ez * ez) - hd - fabsf(a.w), k));
-    }
-    p += 2 * (n.nc + n.nzc);
-    for (int i = 0; i < n.ncb + n.nzb; i++, k++) {
-        const float4 c0 = __ldg(p + 4 * i), c1 = __ldg(p + 4 * i + 1), c2 = __ldg(p + 4 * i + 2), c3 = __ldg(p + 4 * i + 3);
-        const float dx = cx - c0.x, dy = cy - c0.y, dz = cz - c0.z;
-        auto term = [&](float ax, float ay, float az, float h) {
-            return fmaxf(fabsf(ax * dx + ay * dy + az * dz) - h - (fabsf(ax) * hx + fabsf(ay) * hy + fabsf(az) * hz), 0.0f);
-        };
-        const bool up = i >= n.ncb;
-        const float t1 = term(c1.x, c1.y, up ? 0.0f : c1.z, c0.w), t2 = term(c2.x, c2.y, up ? 0.0f : c2.z, c1.w),
-                    t3 = up ? term(0.0f, 0.0f, 1.0f, c2.w) : term(c3.x, c3.y, c3.z, c2.w);
-        insert(key, bound_key(sqrtf(t1 * t1 + t2 * t2 + t3 * t3), k));
-    }
-    const unsigned next = key[15] >> 8;
-    const_cast<uint8_t *>(s_g.near_)[cell] = (uint8_t)(key[0] >> 8);
-    // the listed ones by obstacle number (a bitonic network; unused entries last)
-    key[15] = 0xFFFFu;
-#pragma unroll
-    for (int i = 0; i < 16; i++) key[i] = ((key[i] & 255u) << 8) | (key[i] >> 8);
-#pragma unroll
-    for (int size = 2; size <= 16; size <<= 1)
-#pragma unroll
-        for (int step = size >> 1; step > 0; step >>= 1)
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const int j = i ^ step;
-                if (j > i) {
-                    const unsigned lo = min(key[i], key[j]), hi = max(key[i], key[j]);
-                    key[i] = (i & size) ? hi : lo;
-                    key[j] = (i & size) ? lo : hi;
-                }
-            }
-    unsigned lb[4], num[4];
-#pragma unroll
-    for (int w = 0; w < 4; w++) {
-        lb[w] = num[w] = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const unsigned v = 4 * w + i == 15 ? 0xFF00u | next : key[4 * w + i];
-            lb[w] |= (v & 255u) << (8 * i);
-            num[w] |= (v >> 8) << (8 * i);
-        }
-    }
-    uint4 *L = const_cast<uint4 *>(s_g.list) + 2 * (size_t)cell;
-    L[0] = make_uint4(lb[0], lb[1], lb[2], lb[3]);
-    L[1] = make_uint4(num[0], num[1], num[2], num[3]);
+    for (int i = threadIdx.x; i < n.records(); i += kThreads) s_rec[i] = __ldg(s_g.rec + i);
+    __syncthreads();
+    for (int cell = blockIdx.x * kThreads + threadIdx.x; cell < cells; cell += gridDim.x * kThreads) build_cell(s_g, s_rec, n, cell);
 }
-
 }  // namespace
 
 // (the lists, 16-byte entries, follow the header and a multiple of 16 bytes)
@@ -310,7 +318,9 @@ cudaError_t launch_env_grid(EnvGrid header, const float4 *rec, const EnvGrid *wh
 cudaError_t launch_env_grids(const BatchQueryDesc *scenes, int n, int cells, cudaStream_t st)
 {
     for (int first = 0; first < n; first += 65535) {
-        const dim3 grid((cells + kThreads - 1) / kThreads, std::min(n - first, 65535));
+        // (many scenes: four cells a thread, for fewer headers and records read)
+        const int per = n >= 64 ? 4 * kThreads : kThreads;
+        const dim3 grid((cells + per - 1) / per, std::min(n - first, 65535));
         k_env_grid<<<grid, kThreads, 0, st>>>(scenes + first, EnvGrid{}, cells);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
