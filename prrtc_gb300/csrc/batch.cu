@@ -354,7 +354,9 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
         if (scene[i] < 0) continue;
         BatchQueryDesc &d = descs[i];
         if (scene[i] == i) {
-            d.env = env_dev + env_rec_off[i];
+            // (null without records: a warp stages anew when the address changes, and
+            // the next scene's records start where this one's would)
+            d.env = d.env_n.records() > 0 ? env_dev + env_rec_off[i] : nullptr;
             if (b->grids && can_have_grid(i)) {
                 d.grid = reinterpret_cast<const EnvGrid *>(b->grids + grid_bytes * own.size());
                 own.push_back(d);

@@ -73,3 +73,25 @@ def test_shared_scenes_hold_one_grid_each(form):
         held = before - torch.cuda.mem_get_info()[0]   # what the context keeps
     own.close()
     assert held < 128 << 20, held
+
+
+def test_a_scene_after_an_empty_one_is_staged(ctx, oracle):
+    """One slot, queries in the order given: the warp that answered a query in
+    an environment without obstacles takes the next scene's, whose records
+    follow at the same place in the batch's memory."""
+    from prrtc_gb300 import scenes
+    from prrtc_gb300.env import Environment
+    first, last = scenes.make_query("panda", "shelf", 80), scenes.make_query("panda", "tabletop", 81)
+    empty, rng = Environment(), np.random.default_rng(4)
+    sc, off = (np.array(v) for v in scenes.LIMITS["panda"])
+    q = (rng.random((400, 7)) * sc + off).astype(np.float32)
+    free = q[oracle.check("panda", last.env, q) == 1]
+    queries = [(first.env, first.start, first.goal)]
+    for i in range(20):
+        queries += [(empty, first.start, first.goal), (last.env, free[2 * i], free[2 * i + 1])]
+    got = _answers(ctx, queries, max_active=1, admission=1, warps_per_block=1, blocks_per_sm=1)
+    mine = np.flatnonzero(got["solved"])[1:]
+    assert sum(queries[i][0] is last.env for i in mine) >= 10
+    for i in mine:
+        p = got["paths"][i][:got["path_rows"][i]]
+        assert oracle.check_edges("panda", queries[i][0], p[:-1], p[1:], 32).all(), i
