@@ -282,9 +282,11 @@ typedef struct prrtc_batch_settings {
                                         0 tightest first (smallest clearance of start or goal to an
                                         obstacle, computed on the GPU at create: the hard queries
                                         start early and no longer set the batch's end); 1 as given */
-    uint32_t idle_wait_limit;        /* polls (about 256 ns each) a warp with no work to take makes
+    uint32_t idle_wait_limit;        /* polls (256 ns and a look at the slots, 1 us or more) a warp
+                                        with no work to take makes
                                         before it gives up and the run ends with PRRTC_ECUDA and
-                                        stats.error = 1 (0: 2^22, about a second) */
+                                        stats.error = 1 (0: 2^26, minutes: far above the time that
+                                        attempts at their worker cap keep other warps waiting) */
     int shared_frames;               /* 1: the checker keeps its forward-kinematics frames in each
                                         warp's shared memory; 0: in local memory (cached by L1) */
     int rounds_per_header;           /* batches of 32 samples a warp may draw under one read of the

@@ -427,7 +427,7 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
     P.max_workers = settings->max_workers_per_attempt > 0 ? settings->max_workers_per_attempt : 1 << 30;
     P.bases_lanes = c->bases_lanes;
     P.restart_after_ns = settings->restart_after_ns ? settings->restart_after_ns : 10000000ull;
-    P.idle_limit = settings->idle_wait_limit ? settings->idle_wait_limit : (1u << 22);
+    P.idle_limit = settings->idle_wait_limit ? settings->idle_wait_limit : (1u << 26);
     P.shared_frames = settings->shared_frames ? 1 : 0;
     P.sub_rounds = settings->rounds_per_header > 0 ? std::min(settings->rounds_per_header, 64) : 4;
     // pRRTC stops a query when any of its num_new_configs lanes passes max_iters
