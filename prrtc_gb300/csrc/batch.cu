@@ -223,6 +223,19 @@ extern "C" void prrtc_batch_settings_default(prrtc_batch_settings *s)
     prrtc_settings_default(&s->plan);
 }
 
+// What a batch holds, and the batch (caller holds c->mu with the device current).
+static void release_batch(Ctx *c, prrtc_batch *b)
+{
+    cudaStreamSynchronize(c->stream);
+    if (b->graph) cudaGraphExecDestroy(b->graph);
+    if (b->ev0) cudaEventDestroy(b->ev0);
+    if (b->ev1) cudaEventDestroy(b->ev1);
+    cudaFree(b->blob);
+    give_back_grids(c, b->grids);
+    give_back_arena(c, b->arena);
+    delete b;
+}
+
 extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, const prrtc_query *queries, int n,
                                            const prrtc_batch_settings *settings, prrtc_batch **out)
 {
@@ -335,7 +348,7 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
         return c->fail(PRRTC_ENOMEM, "batch_create: cannot allocate %zu bytes", off);
     }
     if ((s = take_arena(c, D, cap, slots, &b->arena))) {
-        prrtc_batch_free(ctx, b);
+        release_batch(c, b);
         return s;
     }
     // host scenes get a clearance grid each, if there is room left for them
@@ -376,7 +389,7 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
                                         c->stream), "batch grids")))) ||
         (s = c->cuda(cudaEventCreate(&b->ev0), "event")) || (s = c->cuda(cudaEventCreate(&b->ev1), "event")) ||
         (s = c->cuda(cudaStreamSynchronize(c->stream), "batch upload"))) {
-        prrtc_batch_free(ctx, b);
+        release_batch(c, b);
         return s;
     }
     // admission order: tightest start/goal clearance first (longest expected
@@ -386,7 +399,7 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
         std::vector<float> score(n);
         if ((s = query_clearance(c, robot, reinterpret_cast<const BatchQueryDesc *>(base + o_desc),
                                  reinterpret_cast<const float *>(base + o_cfg), n, score.data()))) {
-            prrtc_batch_free(ctx, b);
+            release_batch(c, b);
             return s;
         }
         std::vector<int> order(n);
@@ -394,7 +407,7 @@ extern "C" prrtc_status prrtc_batch_create(prrtc_ctx *ctx, prrtc_robot robot, co
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return score[x] < score[y]; });
         order_dev = reinterpret_cast<int *>(base + o_order);
         if ((s = c->cuda(cudaMemcpy(order_dev, order.data(), n * sizeof(int), cudaMemcpyHostToDevice), "batch order"))) {
-            prrtc_batch_free(ctx, b);
+            release_batch(c, b);
             return s;
         }
     }
@@ -597,18 +610,9 @@ extern "C" prrtc_status prrtc_batch_free(prrtc_ctx *ctx, prrtc_batch *b)
 {
     Ctx *c = Ctx::of(ctx);
     if (!c || !b) return PRRTC_EINVAL;
-    {
-        std::lock_guard<std::mutex> g(c->mu);
-        cudaSetDevice(c->device);
-        cudaStreamSynchronize(c->stream);
-        if (b->graph) cudaGraphExecDestroy(b->graph);
-        if (b->ev0) cudaEventDestroy(b->ev0);
-        if (b->ev1) cudaEventDestroy(b->ev1);
-        cudaFree(b->blob);
-        give_back_grids(c, b->grids);
-        give_back_arena(c, b->arena);
-    }
-    delete b;
+    std::lock_guard<std::mutex> g(c->mu);
+    cudaSetDevice(c->device);
+    release_batch(c, b);
     return PRRTC_OK;
 }
 
