@@ -191,7 +191,7 @@ extern "C" prrtc_status prrtc_path_cost_grad(prrtc_ctx *ctx, prrtc_robot robot, 
         (s = c->device_view(cost, rows * sizeof(float), 1, false, &dcost)) ||
         (s = c->device_view(grad, rows * M.dof * sizeof(float), 2, false, &dgrad)))
         return s;
-    if ((s = c->cuda(ops->path_cost_grad(M, c->clearance->envs, (int64_t)rows, waypoints, (const float *)dq, margin,
+    if ((s = c->cuda(ops->path_cost_grad(M, c->clearance->envs, n_paths, waypoints, max_rec, (const float *)dq, margin,
                                          (float *)dcost, (float *)dgrad, c->stream), "path_cost_grad: launch")))
         return s;
     c->launches++;

@@ -177,10 +177,11 @@ __device__ __forceinline__ bool env_near(const EnvGrid *g, float3 c, float r)
 // configuration (dof floats).  Returns the cost to all four lanes and, in gr,
 // dC/dq of the joints at table positions l, l + 4, ... (l: lane within the
 // four).  Configurations out of the kinematics' range (not finite, beyond
-// 100 rad in sum) are left to the one-thread form.
+// 100 rad in sum) are left to the one-thread form: here, on one of the four
+// lanes, or with `left` by the caller, who is told.
 template <class Gen>
 __device__ double eval(EvalScratch<Gen::kFrames - 1> &S, const ClrModel &M, const ClrEnv &e, const float *q, bool active,
-                       float mf, double (&gr)[(Gen::kFrames + 2) / 4])
+                       float mf, double (&gr)[(Gen::kFrames + 2) / 4], bool *left = nullptr)
 {
     constexpr int NJ = Gen::kFrames - 1, SLOTS = (Gen::kFrames + 2) / 4;
     constexpr unsigned FULL = 0xffffffffu;
@@ -369,7 +370,9 @@ __device__ double eval(EvalScratch<Gen::kFrames - 1> &S, const ClrModel &M, cons
     cost += __shfl_xor_sync(FULL, cost, 1);
     cost += __shfl_xor_sync(FULL, cost, 2);
 
-    if (__any_sync(FULL, far)) {
+    if (left) {
+        *left = far;
+    } else if (__any_sync(FULL, far)) {
         // table order, through the shared scratch
         if (far && l == 0) {
             float g[kClrMaxJoints];
@@ -391,7 +394,8 @@ __device__ double eval(EvalScratch<Gen::kFrames - 1> &S, const ClrModel &M, cons
 
 }  // namespace clr
 
-// Every waypoint of every path, four lanes each.
+// Every waypoint of every path, four lanes each; those out of the kinematics'
+// range then by a thread each, next to one another.
 template <class Gen>
 __global__ void __launch_bounds__(64) k_path_cost_grad(ClrModel M, const ClrEnv *__restrict__ envs, int64_t rows,
                                                       int waypoints, const float *__restrict__ q, float margin,
@@ -399,17 +403,51 @@ __global__ void __launch_bounds__(64) k_path_cost_grad(ClrModel M, const ClrEnv 
 {
     constexpr int NJ = Gen::kFrames - 1, SLOTS = (Gen::kFrames + 2) / 4;
     __shared__ clr::EvalScratch<NJ> s_eval[16];
+    __shared__ bool s_left[16];
     const int l = threadIdx.x & 3;
-    const int64_t row = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 2);
+    const int64_t first = (int64_t)blockIdx.x * 16;
+    int64_t row = first + (threadIdx.x >> 2);
     const bool active = row < rows;
     const ClrEnv e = envs[active ? row / waypoints : 0];
     double gr[SLOTS];
-    const double c = clr::eval<Gen>(s_eval[threadIdx.x >> 2], M, e, q + (active ? row : 0) * M.dof, active, margin, gr);
-    if (!active) return;
-    if (l == 0) cost[row] = (float)c;
+    bool left;
+    const double c = clr::eval<Gen>(s_eval[threadIdx.x >> 2], M, e, q + (active ? row : 0) * M.dof, active, margin, gr, &left);
+    if (active && !left) {
+        if (l == 0) cost[row] = (float)c;
 #pragma unroll
-    for (int t = 0; t < SLOTS; t++)
-        if (l + 4 * t < NJ) grad[row * M.dof + M.joints[l + 4 * t].q] = (float)gr[t];
+        for (int t = 0; t < SLOTS; t++)
+            if (l + 4 * t < NJ) grad[row * M.dof + M.joints[l + 4 * t].q] = (float)gr[t];
+    }
+    if (!__syncthreads_or(left)) return;
+    if (l == 0) s_left[threadIdx.x >> 2] = left;
+    __syncthreads();
+    if (threadIdx.x >= 16 || !s_left[threadIdx.x]) return;
+    row = first + threadIdx.x;
+    float g[kClrMaxJoints];
+    cost[row] = clr::cost_grad(M, envs[row / waypoints], q + row * M.dof, margin, 1.0f, g);
+    for (int d = 0; d < M.dof; d++) grad[row * M.dof + d] = g[d];
+}
+
+// The same with a thread per waypoint, blocks of 64 waypoints of one path and
+// the path's obstacles in shared memory: for robots with fewer leaves than four
+// lanes (the sphere robot's 256 paths among 32 obstacles 217 us a call, 257
+// with four lanes).
+template <class Gen>
+__global__ void __launch_bounds__(64) k_path_cost_grad_one(ClrModel M, const ClrEnv *__restrict__ envs, int waypoints,
+                                                          const float *__restrict__ q, float margin,
+                                                          float *__restrict__ cost, float *__restrict__ grad)
+{
+    extern __shared__ float4 s_env[];
+    __shared__ unsigned long long s_bar;
+    const int path = blockIdx.y;
+    const ClrEnv pe = envs[path];
+    stage_env_bulk(s_env, pe.rec, pe.n.records(), &s_bar);
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= waypoints) return;
+    const size_t row = (size_t)path * waypoints + w;
+    float g[kClrMaxJoints];
+    cost[row] = clr::cost_grad(M, ClrEnv{s_env, pe.n}, q + row * M.dof, margin, 1.0f, g);
+    for (int d = 0; d < M.dof; d++) grad[row * M.dof + d] = g[d];
 }
 
 }  // namespace prrtc

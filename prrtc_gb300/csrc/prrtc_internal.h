@@ -234,8 +234,8 @@ struct RobotOps {
     cudaError_t (*solve_plain)(const PlainParams &, int threads, cudaStream_t);
     cudaError_t (*solve_batch)(const BatchParams &, int blocks, int warps_per_block, cudaStream_t);
     int (*batch_occupancy)(int warps_per_block, int env_records, int shared_frames);   // resident blocks per SM
-    cudaError_t (*path_cost_grad)(const ClrModel &, const ClrEnv *envs, int64_t rows, int waypoints, const float *q,
-                                  float margin, float *cost, float *grad, cudaStream_t);
+    cudaError_t (*path_cost_grad)(const ClrModel &, const ClrEnv *envs, int n_paths, int waypoints, int max_records,
+                                  const float *q, float margin, float *cost, float *grad, cudaStream_t);
     cudaError_t (*smooth_paths)(const ClrLaunch &, size_t env_bytes, cudaStream_t);
     cudaError_t (*goal_flags)(const LaunchEnv &, const GoalQuery &, uint8_t *flags, cudaStream_t);
 };

@@ -611,11 +611,18 @@ struct RobotKernels {
             k_goal_flags<Gen, EveryCheckCtx><<<blocks, 128, smem, st>>>(le.rec, le.counts, nullptr, g, flags);
         return cudaGetLastError();
     }
-    static cudaError_t path_cost_grad(const ClrModel &M, const ClrEnv *envs, int64_t rows, int waypoints, const float *q,
-                                      float margin, float *cost, float *grad, cudaStream_t st)
+    static cudaError_t path_cost_grad(const ClrModel &M, const ClrEnv *envs, int n_paths, int waypoints, int max_records,
+                                      const float *q, float margin, float *cost, float *grad, cudaStream_t st)
     {
-        if (rows <= 0) return cudaSuccess;
-        k_path_cost_grad<Gen><<<(unsigned)((rows + 15) / 16), 64, 0, st>>>(M, envs, rows, waypoints, q, margin, cost, grad);
+        if (n_paths <= 0) return cudaSuccess;
+        if constexpr (Gen::kNumSpheres < 4) {
+            k_path_cost_grad_one<Gen><<<dim3((waypoints + 63) / 64, n_paths), 64, (size_t)max_records * sizeof(float4), st>>>(
+                M, envs, waypoints, q, margin, cost, grad);
+        } else {
+            (void)max_records;
+            const int64_t rows = (int64_t)n_paths * waypoints;
+            k_path_cost_grad<Gen><<<(unsigned)((rows + 15) / 16), 64, 0, st>>>(M, envs, rows, waypoints, q, margin, cost, grad);
+        }
         return cudaGetLastError();
     }
     static cudaError_t smooth_paths(const ClrLaunch &P, size_t env_bytes, cudaStream_t st)
