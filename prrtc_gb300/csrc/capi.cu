@@ -190,7 +190,7 @@ prrtc_status prrtc_destroy(prrtc_ctx *ctx)
         c->release_planner_state();
         release_arena(c);
         release_clearance_state(c);
-        if (c->env_pool) cudaMemPoolDestroy(c->env_pool);
+        for (auto &b : c->env_blocks) cudaFree(b.ptr);
         cudaFree(c->work_dev);
         for (cudaEvent_t ev : c->kev)
             if (ev) cudaEventDestroy(ev);
@@ -266,42 +266,36 @@ prrtc_status prrtc_robot_limits(prrtc_robot robot, float *scale, float *offset)
 // upload 40 / 57 / 71 us and the free 9 / 15 / 21 us.
 static constexpr int kEnvCells = 16384;
 
-// Environments with a grid come from a memory pool of the context that keeps up
-// to this much between them: allocating and freeing 0.5 MB took 12 and 10 us
-// from the driver, 1 and 1 from the pool.  Memory in use when the context is
-// destroyed stays until its environment is freed.
-static constexpr uint64_t kEnvKept = (uint64_t)64 << 20;
+// The memory of up to this many freed environments with grids (0.5 MB each) is
+// kept for the context's next ones: allocating and freeing it took 12 and 10 us.
+static constexpr size_t kEnvBlocks = 32;
+static constexpr size_t kEnvBlockStep = 8192;   // sizes are rounded up, so that scenes of a kind fit one another's blocks
 
 static bool env_alloc(Ctx *c, Env *e, size_t bytes)
 {
-    if (!c->env_pool_tried) {
-        c->env_pool_tried = true;
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = c->device;
-        uint64_t kept = kEnvKept;
-        if (cudaMemPoolCreate(&c->env_pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(c->env_pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) {
-            cudaGetLastError();
-            if (c->env_pool) cudaMemPoolDestroy(c->env_pool);
-            c->env_pool = nullptr;
+    bytes = (bytes + kEnvBlockStep - 1) / kEnvBlockStep * kEnvBlockStep;
+    e->device = c->device;
+    e->bytes = bytes;
+    for (size_t i = 0; i < c->env_blocks.size(); i++)
+        if (c->env_blocks[i].bytes == bytes) {
+            e->dev = static_cast<float4 *>(c->env_blocks[i].ptr);
+            c->env_blocks[i] = c->env_blocks.back();
+            c->env_blocks.pop_back();
+            return true;
         }
-    }
-    e->pooled = c->env_pool && cudaMallocFromPoolAsync((void **)&e->dev, bytes, c->env_pool, c->stream) == cudaSuccess;
-    if (e->pooled) return true;
-    cudaGetLastError();
     if (cudaMalloc(&e->dev, bytes) == cudaSuccess) return true;
     cudaGetLastError();
     e->dev = nullptr;
     return false;
 }
 
+// Caller holds c->mu; the context's stream is idle.  (Every call that reads an
+// environment returns when its work is done, so no other context's work reads
+// it either.)
 static void env_release(Ctx *c, Env *e)
 {
-    // (every call that reads an environment returns when its work is done)
-    if (e->pooled)
-        cudaFreeAsync(e->dev, c->stream);
+    if (e->grid && e->device == c->device && c->env_blocks.size() < kEnvBlocks)
+        c->env_blocks.push_back(Ctx::Buf{e->dev, e->bytes});
     else
         cudaFree(e->dev);
     delete e;

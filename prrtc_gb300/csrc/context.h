@@ -13,7 +13,8 @@ struct Env {
     EnvCounts counts{};
     float4 *dev = nullptr;           // packed records on the device, followed by the clearance grid
     const EnvGrid *grid = nullptr;
-    bool pooled = false;             // dev is from a context's env_pool, else from cudaMalloc
+    size_t bytes = 0;                // allocated at dev
+    int device = 0;
     std::vector<float4> host;        // the same records on the host
     uint32_t num_cylinders = 0;      // accepted, never checked (as the reference)
 };
@@ -74,8 +75,7 @@ struct Ctx {
     float *bases = nullptr;                 // Halton prime bases per sampling lane [lanes][16]
     int bases_lanes = 0;
     struct Arena *arena = nullptr;          // batched-planner arena kept between batches
-    cudaMemPool_t env_pool = nullptr;       // environments with grids (prrtc_env_upload)
-    bool env_pool_tried = false;
+    std::vector<Buf> env_blocks;            // memory of freed environments, for the next ones (at most kEnvBlocks)
     Buf grids;                              // clearance grids' memory kept between batches (at most kGridsKept)
     bool grids_in_use = false;              // by a live batch
     unsigned long long *work_dev = nullptr; // [2] FLOPs, configurations (prrtc_work_counters)

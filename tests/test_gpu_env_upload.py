@@ -40,7 +40,7 @@ def test_environments_freed_in_any_order_and_used_by_other_contexts(ctx):
 
 
 def test_memory_kept_for_environments_is_bounded():
-    """400 environments of 0.5 MB, all held, then freed: at most the pool's 64 MB stay, and nothing after the context."""
+    """400 environments of 0.5 MB, all held, then freed: at most 32 of them stay, and nothing after the context."""
     import torch
     from prrtc_gb300 import Context, scenes
     torch.cuda.synchronize()
@@ -54,6 +54,6 @@ def test_memory_kept_for_environments_is_bounded():
         h.free()
     own.validate_configs("panda", scenes.tabletop_scene(0), _configs(10))
     kept = before - free()
-    assert kept <= 96 << 20, kept
+    assert kept <= 40 << 20, kept
     own.close()
     assert free() >= before - (8 << 20)
