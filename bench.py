@@ -16,7 +16,9 @@ JSON line (the contract this repository's driver reads):
   plain      the drop-in single-query form (prrtc_solve) on a sample of the
              same queries, one at a time
   roofline   the planner kernel's algorithmic FP32 FLOPs (counted in-kernel:
-             canonical FK + the reference checker's executed tests x weights)
+             canonical FK + the tests that the reference's checker makes x
+             weights; the fast checker knows most of their answers from
+             bounds, so this is a rate of answers, not of arithmetic done)
              per launch / launch time, against the device's measured FP32 FMA
              peak (neither the HBM nor the tensor roof applies: the validator
              is SIMT FP32 work on L1/L2-resident data)

@@ -231,9 +231,9 @@ __device__ __forceinline__ Ctx make_ctx(const EnvView &view, float pad, volatile
 // gives round r the points 32 r + lane + 1; interleaved order gives it
 // lane * R + r + 1, so the first round already samples the whole edge at
 // stride R.  Adds the work done to work[0] (FLOPs) and work[1] (points).  A
-// called function: inlined where edges are extended and connected, with both
-// kinds of frame storage, the checker took the kernel's four copies of it to
-// 168 registers (12 warps per SM).
+// called function, so that the kernel holds each form of the checker once:
+// inlined where edges are extended and where they are connected, 1024 tabletop
+// queries took 4.02 instead of 3.19 ms and 4096 shelf queries 107 instead of 95.
 template <class Gen, class Ctx>
 __device__ __noinline__ bool warp_validate(WarpScratch<Gen::kDof> &W, float4 *frames, int g, int interleave, float pad,
                                            unsigned long long *work)

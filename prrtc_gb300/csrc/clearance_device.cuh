@@ -14,13 +14,15 @@
 // no gradient to follow out of it.
 //
 // Precision: every sphere-obstacle and sphere-sphere term is first screened
-// in float32 (the bulk of the work); the few terms the screen keeps, the
-// forward kinematics and the adjoint sweep run in float64, so the result
+// in float32 (the bulk of the work); the few terms the screen keeps and the
+// forces run in float64, the forward kinematics in float64 in the one-thread
+// form below and in pairs of floats (2^-44) in the four-lane form
+// (clearance_eval.cuh), so the result
 // matches a float64 evaluation to ~1e-7 even for terms a fraction of a
 // millimetre inside the margin (float32 coordinates near 1 m are only good
 // to 6e-8 m, a 4e-4 relative error on such a term).
 //
-// The adjoint recomputes forward kinematics rather than keeping per-link
+// The one-thread form's adjoint recomputes forward kinematics rather than keeping per-link
 // transforms from a forward pass.  Each active term becomes a force
 // g = dC/dc on a sphere centre c; per joint j the forces G_j and the moments
 // M_j = sum (c - o_j) x g about the joint's origin o_j are summed, then

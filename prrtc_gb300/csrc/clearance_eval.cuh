@@ -64,8 +64,9 @@ __device__ __forceinline__ Dd operator*(Dd x, float f)
 }
 __device__ __forceinline__ double to_double(Dd x) { return (double)x.h + (double)x.l; }
 
-// Sine and cosine of |q| <= 100 to about 2^-46: q = k pi / 2 + r with pi / 2 in
-// three parts (the first two of 16 bits, so k times them is exact), then the
+// Sine and cosine of |q| <= 100 to 2^-44: q = k pi / 2 + r with pi / 2 in three
+// parts (the first two of 16 bits, so k times them is exact; Cody and Waite's
+// reduction, see near_sincos), then the
 // Taylor series of r, |r| <= pi / 4, up to r^15 / r^16, the coefficients down to
 // 1 / 7! and 1 / 8! in pairs.
 __device__ __forceinline__ Dd coef(double c) { return Dd{(float)c, (float)(c - (double)(float)c)}; }

@@ -270,11 +270,16 @@ __host__ __device__ __forceinline__ int env_cost_all(const EnvCounts &n)
 
 // Sphere against obstacle k: 0 no hit, 1 hit, 2 too near contact to tell
 // here.  The distance is the reference test's; what is left to the exact test
-// is a band around contact wider than any rounding: 3e-6 m (two forms of the
-// kinematics differ by less than 1.5e-6 m, and the distances of spheres that
-// near by less), and for capsules and boxes 5e-7 of the offset from the
-// obstacle's origin, whose products round by as much.  So verdicts do not
-// depend on how two copies of a formula are contracted.
+// is a band around contact wider than any rounding: 3e-6 m, and for capsules
+// and boxes 5e-7 of the offset from the obstacle's origin, whose products round
+// by as much.  So verdicts do not depend on how two copies of a formula are
+// contracted.  What the 3e-6 m cover: a centre's error in one form of the
+// kinematics is at most the sum over the joints of a chain (7 or 8; Baxter's 14
+// are two chains of 7) of the sine's error, 1.0e-7, times the reach, 1.2 m, and
+// of the products' rounding, about as much: 1.7e-6 m if all added up.  Measured
+// over 4.7 M configurations per robot, in the joint limits and up to 100 rad in
+// sum: a centre is within 3.6e-7 m of float64 in either form, the two forms are
+// within 5.0e-7 m of one another, and distances of pairs within 3.5e-7 m.
 constexpr float kGridReach = 8.0f;
 __device__ __forceinline__ int near_verdict(float d2, float rs, float band = 3e-6f)
 {
@@ -383,9 +388,10 @@ __device__ __forceinline__ int grid_hit(const EnvView &e, float x, float y, floa
 }
 
 // Sphere against every obstacle: by the grid where there is one.  Every
-// obstacle for every sphere was two thirds of a check; 2^20 random
-// configurations on the Panda shelf scene (41 obstacles) take 1.01 ms instead
-// of 1.86, 200 003 Baxter ones among 72 obstacles 0.66 ms instead of 1.20.
+// obstacle for every sphere was two thirds of a check: with this alone, 2^20
+// random configurations on the Panda shelf scene (41 obstacles) went from 1.86
+// to 1.01 ms, 200 003 Baxter ones among 72 obstacles from 1.20 to 0.66 (0.79 and
+// 0.48 with the fast form of near_check.cuh in front of it).
 static __device__ __noinline__ int env_hit(const EnvView e, float x, float y, float z, float r)
 {
     const int h = e.grid ? grid_hit(e, x, y, z, r) : -1;
@@ -556,7 +562,9 @@ __device__ __forceinline__ Frame frame_at(const SharedFrames F, int i)
 // reference checker's verdicts; planners may inflate every sphere by pad
 // (a certified margin) and share a flag through which any lane's collision
 // ends the other lanes' work on the same edge.  `work` accumulates the
-// algorithmic FLOPs of the primitive tests executed (reference weights).
+// algorithmic FLOPs of the primitive tests that the reference's checker makes
+// on the configuration (reference weights), whether they are made here or
+// known from a bound.
 struct CheckCtx {
     static constexpr bool kSharedFrames = false;   // table-form frames in a local array
     static constexpr bool kInlineExact = false;    // the exact form (near_check.cuh) as a called function

@@ -37,10 +37,11 @@ struct alignas(16) NearPairBlock {
     int row;
 };
 
-// Sine and cosine to 1e-7 for |x| <= 100: x minus a multiple of pi / 2 (in three
-// parts, the first two products exact), then the Taylor series up to r^9 / r^10.
-// The exact form has the library's; the two forms' centres differ by less
-// than 1.5e-6 m (half of near_verdict's band).
+// Sine and cosine to 1.75 x 2^-24 (1.0e-7) for |x| <= 100: x minus a multiple of
+// pi / 2 in three parts, the first two products exact (the reduction of W. J. Cody
+// and W. Waite, "Software Manual for the Elementary Functions", 1980), then the
+// Taylor series up to r^9 / r^10.  The exact form has the library's; the two
+// forms' centres differ by at most 5.0e-7 m (near_verdict).
 __device__ __forceinline__ void near_sincos(float x, float *s, float *c)
 {
     const float k = rintf(x * 0.636619772f);
@@ -239,6 +240,8 @@ __device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const St
     T::frames(q.q, F, G);
 #pragma unroll 1
     for (int w = 0; w < T::kWords; w++) {
+        // (the lanes that are together here, each with its own bits among `todo`:
+        // verdicts do not depend on which lanes are, the speed does)
         const unsigned word = m.marked[w];
         unsigned todo = __reduce_or_sync(__activemask(), word);
 #pragma unroll 1

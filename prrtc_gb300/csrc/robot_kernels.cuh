@@ -39,11 +39,11 @@ __device__ __forceinline__ void add_work(unsigned long long *work, unsigned long
 
 // Launch bounds of the stand-alone configuration checker, per robot: by
 // default at most 64 registers (128-thread blocks, 8 per SM): the marking code
-// spills a little but 32 resident warps per SM hide its waits better.  A
-// million random Panda configurations on a shelf scene: 826 us at 64
-// registers, 1142 at 80, 1212 at 96, 1040 at 128 (before the exact form was
-// cut down to marked steps and the sines were inlined; 782 us now).  A robot
-// file may specialise it.
+// spills but 32 resident warps per SM hide its waits better.  Random
+// configurations on a shelf scene at 8 / 6 / 5 / 4 blocks per SM (64 / 80 / 96 /
+// 128 registers): a million of Panda 798 / 846 / 903 / 994 us, 200 003 of Fetch 522
+// / 523 / 563 / 585, of Baxter 460 / 421 / 454 / 461; a hundred take the same
+// within 5 us.  A robot file may specialise it.
 template <class Gen>
 struct ValidateLaunch {
     static constexpr int kMaxThreads = 128, kMinBlocks = 8;
@@ -101,7 +101,10 @@ struct LongEdges {
 // Chunk-major order: an edge's chunks run far apart, so that a later chunk
 // mostly finds the earlier ones' answer.  An edge of at most 32 points has one
 // warp, which writes its answer (no memset before the launch: 3 us of a call
-// that takes 25 to 40).
+// that takes 25 to 40).  MinBlocks: 6 (at most 80 registers); 2^14 edges of 128
+// points on a shelf scene at 8 / 6 / 4 blocks and unbounded: Panda 607 / 607 / 602 /
+// 603 us, Fetch 973 / 965 / 971 / 961; Baxter's of 32 points 828 / 895 / 966 / 983,
+// a thousand of 50 points 152 / 149 / 120 / 124.
 template <class Gen, class Ctx, int MinBlocks>
 __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
                                                         const EnvGrid *grid,
@@ -239,7 +242,8 @@ __global__ void __launch_bounds__(128) k_goal_flags(const float4 *__restrict__ e
 // 16 bytes a sphere (1.1 KB a Panda configuration).  Written from each thread's
 // registers the rows of neighbouring lanes lie a configuration apart, half a
 // sector per store; so the warp's rows are put together in shared memory (lane
-// strides of 276 and 500 words: no bank conflicts) and leave as one bulk copy of
+// strides of 276, 500 and 400 words: a store of 16 bytes a lane takes its four
+// passes for Panda and Fetch, Baxter's lanes meet in the same banks) and leave as one bulk copy of
 // the TMA engine, 32 configurations being one run of memory.  100 000 Panda
 // configurations (113 MB): 50 us a call before, 30 now (12 of them the call).
 template <class Gen>
