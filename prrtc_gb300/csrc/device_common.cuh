@@ -466,12 +466,13 @@ static __device__ __noinline__ int self_pairs(const Frame Tab, const LeafPair *_
 // tables, making the same ctx calls in the same order (same verdicts, same
 // counts).  Frames are indexed by joint config index + 1; F[0] is the world.
 
-struct alignas(8) GenSched {   // (a lone warp waits for each cache line of the table)
-    short step;        // environment group k: k; self group k: -1 - k
+struct GenStep {
+    int kind;          // 0 environment group, 1 self group
+    int index;
+};
+struct GenSched : GenStep {
     short env, self;   // sphere-environment and gate-pair tests of the steps up to and with this one, none hit
-    short tests;       // environment: sphere tests of this step when nothing hits; self: its leaf pairs
-    __device__ __forceinline__ bool environment() const { return step >= 0; }
-    __device__ __forceinline__ int group() const { return step >= 0 ? step : -1 - step; }
+    int tests;         // environment: sphere tests of this step when nothing hits; self: its leaf pairs
 };
 struct GenEnvGroup {
     int gate;             // gating sphere: index into the gate centres, -1 none
@@ -679,6 +680,16 @@ struct StepMarks {
 };
 struct AllSteps {};   // in the place of the marks: every step
 
+// The schedule as either reads it.  (Without the counts it is half as long: a
+// lone warp that makes every step waits for each cache line of the table, 12 us
+// of Baxter's 190.)
+template <int W>
+__device__ __forceinline__ const GenSched *schedule(const StepMarks<W> &, const GenSched *counted, const GenStep *)
+{
+    return counted;
+}
+__device__ __forceinline__ const GenStep *schedule(AllSteps, const GenSched *, const GenStep *steps) { return steps; }
+
 // G: the world centres of the gate spheres, computed with the frames (the
 // same xform as a leaf's, so verdicts do not change).  The steps that are not
 // made count as the reference makes them.  (Making all 388 of them cost a Baxter
@@ -699,9 +710,9 @@ __device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restri
             if (s >= nsched) break;
             const GenSched e = sched[s];
             bool hit = false;
-            if (e.environment()) {
+            if (e.kind == 0) {
                 known += cost * e.tests;
-                const GenEnvGroup g = eg[e.group()];
+                const GenEnvGroup g = eg[e.index];
                 bool go = true;
                 if (g.gate >= 0) {
                     const float4 c = G[g.gate];
@@ -716,7 +727,7 @@ __device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restri
                 ctx.work += kFlopPair * e.tests;
             } else {
                 known += kFlopPair;
-                const GenSelfGroup g = sg[e.group()];
+                const GenSelfGroup g = sg[e.index];
                 const float4 a = G[g.ga], b = G[g.gb];
                 if (ctx.pair_hit(a.x - b.x, a.y - b.y, a.z - b.z, a.w + b.w))
                     for (int k = g.first_block; k < g.first_block + g.nblocks && !hit; k++) {
@@ -736,7 +747,7 @@ __device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restri
 }
 
 template <class Frames, class Ctx>
-__device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restrict__ G, const GenSched *__restrict__ sched,
+__device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restrict__ G, const GenStep *__restrict__ sched,
                                           int nsched,
                                           const GenEnvGroup *__restrict__ eg, const GenLeafBlock *__restrict__ lb,
                                           const float4 *__restrict__ leaves, const GenSelfGroup *__restrict__ sg,
@@ -744,9 +755,9 @@ __device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restri
                                           Ctx &ctx, AllSteps)
 {
     for (int s = 0; s < nsched; s++) {
-        const GenSched e = sched[s];
-        if (e.environment()) {
-            const GenEnvGroup g = eg[e.group()];
+        const GenStep e = sched[s];
+        if (e.kind == 0) {
+            const GenEnvGroup g = eg[e.index];
             bool go = true;
             if (g.gate >= 0) {
                 const float4 c = G[g.gate];
@@ -758,7 +769,7 @@ __device__ __noinline__ bool run_schedule(const Frames F, const float4 *__restri
                     if (ctx.env_leaves(frame_at(F, b.frame + 1), leaves + b.first, b.n)) return false;
                 }
         } else {
-            const GenSelfGroup g = sg[e.group()];
+            const GenSelfGroup g = sg[e.index];
             const float4 a = G[g.ga], b = G[g.gb];
             if (ctx.pair_hit(a.x - b.x, a.y - b.y, a.z - b.z, a.w + b.w))
                 for (int k = g.first_block; k < g.first_block + g.nblocks; k++) {

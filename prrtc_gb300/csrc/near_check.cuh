@@ -250,8 +250,8 @@ __device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const St
             if (!(word >> s & 1)) continue;
             const GenSched e = T::steps()[32 * w + s];
             int h = kNearFree, c;
-            if (e.environment()) {
-                const GenEnvGroup gr = T::env_groups()[e.group()];
+            if (e.kind == 0) {
+                const GenEnvGroup gr = T::env_groups()[e.index];
                 bool go = true;
                 if (gr.gate >= 0) {
                     const float4 p = G[gr.gate];
@@ -274,7 +274,7 @@ __device__ __noinline__ unsigned near_resolve(const NearCfg<T::kDof> q, const St
                     }
                 extra -= g->cost * e.tests;
             } else {
-                const GenSelfGroup gr = T::self_groups()[e.group()];
+                const GenSelfGroup gr = T::self_groups()[e.index];
                 const float4 a = G[gr.ga], b = G[gr.gb];
                 const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
                 const int gate = near_verdict(dx * dx + dy * dy + dz * dz, (a.w + b.w) + 2.0f * pad);

@@ -100,12 +100,12 @@ struct LongEdges {
 // edge, waiting for the block's slowest warp was a fifth of the time).
 // Chunk-major order: an edge's chunks run far apart, so that a later chunk
 // mostly finds the earlier ones' answer.  An edge of at most 32 points has one
-// warp, which writes its answer (no memset before the launch: 3 us of a call
+// warp (kOneWarp), which writes its answer (no memset before the launch: 3 us of a call
 // that takes 25 to 40).  MinBlocks: 6 (at most 80 registers); 2^14 edges of 128
 // points on a shelf scene at 8 / 6 / 4 blocks and unbounded: Panda 607 / 607 / 602 /
 // 603 us, Fetch 973 / 965 / 971 / 961; Baxter's of 32 points 828 / 895 / 966 / 983,
 // a thousand of 50 points 152 / 149 / 120 / 124.
-template <class Gen, class Ctx, int MinBlocks>
+template <class Gen, class Ctx, int MinBlocks, bool kOneWarp>
 __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 *__restrict__ env, EnvCounts nc,
                                                         const EnvGrid *grid,
                                                         const float *__restrict__ a, const float *__restrict__ b,
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
     for (int64_t it = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; it < items; it += stride) {
         const int64_t e = it % n;
         const int k = 32 * (int)(it / n) + lane + 1;
-        if (lane == 0) *bad = g > 32 && *(volatile uint8_t *)(out + e) == 0;
+        if (lane == 0) *bad = !kOneWarp && *(volatile uint8_t *)(out + e) == 0;
         __syncwarp();
         if (k <= g && !*bad) {
             float cfg[D];
@@ -142,13 +142,13 @@ __global__ void __launch_bounds__(128, MinBlocks) k_validate_edges(const float4 
             ctx.work = 0;
             if (!Gen::fkcc(cfg, ctx)) {
                 *bad = 1;
-                if (g > 32) out[e] = 0;
+                if (!kOneWarp) out[e] = 0;
             }
             flops += ctx.work + Gen::kFkFlops;
             cfgs++;
         }
         __syncwarp();
-        if (g <= 32 && lane == 0) out[e] = *bad ? 0 : 1;
+        if (kOneWarp && lane == 0) out[e] = *bad ? 0 : 1;
     }
     add_work(work, flops, cfgs);
 }
@@ -547,18 +547,17 @@ struct RobotKernels {
                 k_validate_edges_every<Gen, 0><<<blocks, threads, smem, st>>>(le.rec, le.counts, a, b, n, g, out, le.work);
             return cudaGetLastError();
         }
-        if (chunks > 1) {
-            const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
-            if (e != cudaSuccess) return e;
-        }
         using Long = LongEdges<Gen>;
         const int blocks = grid_for(n * chunks * 32, 128, le.sms, 16);
-        if (chunks >= 4)
-            k_validate_edges<Gen, typename Long::Ctx, Long::kMinBlocks><<<blocks, 128, smem, st>>>(
-                le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
-        else
-            k_validate_edges<Gen, CheckCtx, 6><<<blocks, 128, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
-        return cudaGetLastError();
+        auto launch = [&](auto kernel) {
+            kernel<<<blocks, 128, smem, st>>>(le.rec, le.counts, le.grid, a, b, n, g, out, le.work);
+            return cudaGetLastError();
+        };
+        if (chunks == 1) return launch(k_validate_edges<Gen, CheckCtx, 6, true>);
+        const cudaError_t e = cudaMemsetAsync(out, 1, (size_t)n, st);
+        if (e != cudaSuccess) return e;
+        return chunks < 4 ? launch(k_validate_edges<Gen, CheckCtx, 6, false>)
+                          : launch(k_validate_edges<Gen, typename Long::Ctx, Long::kMinBlocks, false>);
     }
     static cudaError_t fk_spheres(const float *q, int64_t n, float *out, int sms, cudaStream_t st)
     {

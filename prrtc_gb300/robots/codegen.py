@@ -359,7 +359,7 @@ def emit_cuda_checker(m: dict) -> str:
         code.lines.append(f"float4 G[{max(1, len(gate_ids))}];")
         for sidx, gid in gate_ids.items():
             code.lines.append(f"G[{gid}] = gate_centre({fexpr[sp[sidx]['frame']]}, k{R}Gate[{gid}]);")
-        code.lines.append(f"return run_schedule(F.view(), G, k{R}Sched, {len(m['schedule'])}, k{R}EnvGroup, k{R}LeafBlock, k{R}Leaf, "
+        code.lines.append(f"return run_schedule(F.view(), G, schedule(marks, k{R}Sched, k{R}Step), {len(m['schedule'])}, k{R}EnvGroup, k{R}LeafBlock, k{R}Leaf, "
                           f"k{R}SelfGroup, k{R}PairBlock, k{R}Pair, ctx, marks);")
         tcode = code
         code = _Code()              # the straight-line form, if any, goes to its own code
@@ -445,9 +445,12 @@ def emit_cuda_checker(m: dict) -> str:
         for kind, gi in m["schedule"]:
             n = _env_tests(m, gi) if kind == "env" else len(m["self_groups"][gi]["pairs"])
             ne, ns = (ne + n, ns) if kind == "env" else (ne, ns + 1)
-            row = (gi if kind == "env" else -1 - gi, ne, ns, n)
-            assert max(map(abs, row)) < 1 << 15, "GenSched's fields are 16 bits wide"
-            w("    {%d, %d, %d, %d}," % row)
+            assert max(ne, ns) < 1 << 15, "GenSched's counts are 16 bits wide"
+            w(f"    {{{{{0 if kind == 'env' else 1}, {gi}}}, {ne}, {ns}, {n}}},")
+        w("};")
+        w(f"__device__ const GenStep k{R}Step[{len(m['schedule'])}] = {{")
+        for i in range(0, len(m["schedule"]), 8):
+            w("    " + " ".join("{%d, %d}," % (0 if k == "env" else 1, g) for k, g in m["schedule"][i:i + 8]))
         w("};")
         lblocks, eg_rows = [], []
         for gi, g in enumerate(m["env_groups"]):
